@@ -2068,7 +2068,8 @@ public:
         CK(copy_async(lf.data(), r->dsim.lfl, (size_t)n, cudaMemcpyDeviceToHost, stream_));
         CK(cudaStreamSynchronize(stream_));
         for (int i = 0; i < n; i++) {
-            ends4[4 * i] = ln[i]; ends4[4 * i + 1] = lp[i]; ends4[4 * i + 2] = la[i]; ends4[4 * i + 3] = lf[i];
+            ends4[4 * i] = ln[i]; ends4[4 * i + 1] = lp[i]; ends4[4 * i + 2] = la[i];
+            ends4[4 * i + 3] = lf[i] & ~dev::LF_PLAIN;
         }
         return 0;
     }
@@ -2111,7 +2112,7 @@ public:
         for (int i = 0; i < nl; i++) {
             if (d9) for (int k = 0; k < 9; k++) d9[9 * (size_t)i + k] = st[(size_t)k * stride + i];
             if (f3) for (int k = 0; k < 3; k++) f3[3 * (size_t)i + k] = sf[(size_t)k * stride + i];
-            if (flags) flags[i] = fl[i];
+            if (flags) flags[i] = fl[i] & ~dev::LF_PLAIN;
         }
         return 0;
     }

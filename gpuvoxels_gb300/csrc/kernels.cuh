@@ -97,6 +97,11 @@ struct LinkOrient {
     bool switched;    // the mode differs from the previous step's
 };
 
+// A link between two voxels of Fixed materials (VX3 extra): not updated.
+__device__ __forceinline__ bool fixed_link(const Sim& S, int l) {
+    return S.vm[__ldg(S.vmat + __ldg(S.lneg + l))].vx3 & S.vm[__ldg(S.vmat + __ldg(S.lpos + l))].vx3 & VM_FIXED;
+}
+
 // False for a link that is not updated (detached or removed, or between two Fixed voxels).
 __device__ __forceinline__ bool link_orient(const Sim& S, int l, LinkOrient* out) {
     const int ng = __ldg(S.lneg + l), pv = __ldg(S.lpos + l);
@@ -107,7 +112,7 @@ __device__ __forceinline__ bool link_orient(const Sim& S, int l, LinkOrient* out
     // VX3 extras: detached and removed links are no longer updated (VX3_VoxelyzeKernel.cu:565-575),
     // nor are links between two voxels of Fixed materials
     if (fl & LF_GONE) return false;
-    if ((S.flags & SF_FIXEDMAT) && (vN.vx3 & vP.vx3 & VM_FIXED)) return false;
+    if ((S.flags & SF_FIXEDMAT) && fixed_link(S, l)) return false;
     const float tN = S.temp[ng], tP = S.temp[pv];
     const double restLen = half(base_size(vN, tN) + base_size(vP, tP));   // CVX_Link::updateRestLength
     bool small = fl & LF_SMALL, lvv = fl & LF_LVV;
@@ -256,6 +261,38 @@ __device__ __forceinline__ void link_finish(const Sim& S, int l, float dt, const
     S.ss[dn * nv + ng] = 2.0f * strain / (1.0f + ratio);
     S.ss[dp * nv + pv] = 2.0f * strain * ratio / (1.0f + ratio);
 }
+
+}  // namespace GVX_KNS
+}  // namespace gvx
+#include "links_int.cuh"
+namespace gvx {
+namespace GVX_KNS {
+
+// Whether links take the integer-pipe form (links_int.cuh): the exact build does; the FMA build's
+// products contract with their sums on the FP64 pipe.
+#ifdef GVX_CONTRACT
+constexpr bool kLinksInt = false;
+#else
+constexpr bool kLinksInt = true;
+#endif
+
+// The plain form of a whole link update, for a link that the integer-pipe form left (out of line:
+// rare once a body moves).  Sets LF_PLAIN, which keeps the link on this form until plain_retry, so
+// that a body with lasting zeros (an exact symmetry) does not pay for both forms every step.  True
+// when the link's strain diverged.
+__device__ __noinline__ bool link_plain(const Sim& S, int l, float dt) {
+    LinkOrient o;
+    bool div = false;
+    if (link_orient(S, l, &o)) {
+        link_finish(S, l, dt, o, &div);
+        S.lfl[l] |= LF_PLAIN;
+    }
+    return div;
+}
+
+// Steps at which links on the plain form try the integer-pipe form again: the 16th ones, and step 4
+// (of a random creature's links 45-63 % hold an exact zero before step 1, 0.01-0.1 % before step 5).
+__device__ __forceinline__ bool plain_retry(int64_t step) { return step == 4 || (step & 15) == 0; }
 
 // Work-item elements in an order that keeps warps on one code path.  GB300's FP64
 // pipe spends the same cycles on a warp instruction whatever its active lanes, so a
@@ -531,7 +568,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
     for (;;) {
         // this round's links: a full queue, else the claimed chunk (claiming one when it is
         // used up), else what the queues hold at the end
-        int src, cnt = 32;       // src: -1 the chunk, 0 / 1 a queue
+        int src, cnt = 32;       // src: -1 the chunk, 0 / 1 a queue, 2 none left
         if (qn0 >= 32) src = 0;
         else if (qn1 >= 32) src = 1;
         else {
@@ -546,10 +583,14 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
             if (kb < k1) src = -1;
             else if (qn0 > 0) { src = 0; cnt = qn0; }
             else if (qn1 > 0) { src = 1; cnt = qn1; }
-            else break;
+            else src = 2;
         }
+        // the integer-pipe form is long straight-line code: a block's warps keep step through it
+        // (here, and between its three parts below), so that one of them fetches it for all
+        if (kLinksInt ? !__syncthreads_or(src != 2) : src == 2) break;
         int2 e = make_int2(-1, -1);
-        if (src < 0) {
+        if (src == 2) {
+        } else if (src < 0) {
             if (kb + lane < k1) e = __ldg(perm + kb + lane);
             kb += 32;
         } else {
@@ -565,12 +606,28 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
         // have stopped since the grouping was made
         bool act = e.x >= 0 && (unsigned)e.x < (unsigned)n_slots && ctl[e.x].status == 1 && (unsigned)e.y < (unsigned)sims[e.x].nl;
         LinkOrient o;
-        act = act && link_orient(sims[e.x], e.y, &o);
+        IntPipes ip;
+        bool plain = false;      // this link takes the plain form (and is not deferred)
+        if (kLinksInt) {
+            if (act) {
+                const Sim& S = sims[e.x];
+                const uint8_t fl = S.lfl[e.y];
+                act = !(fl & LF_GONE) && !((S.flags & SF_FIXEDMAT) && fixed_link(S, e.y));
+                plain = (fl & LF_PLAIN) && !plain_retry(ctl[e.x].steps);
+                if (act && !plain) {
+                    link_orient_int(ip, S, e.y, fl, &o);
+                    plain = !ip.ok();
+                }
+            }
+        } else {
+            act = act && link_orient(sims[e.x], e.y, &o);
+        }
         if (src < 0) {
-            const unsigned am = __ballot_sync(0xffffffffu, act), sm = __ballot_sync(0xffffffffu, act && o.small);
-            switched += __popc(__ballot_sync(0xffffffffu, act && o.switched));
+            const bool known = act && !plain;
+            const unsigned am = __ballot_sync(0xffffffffu, known), sm = __ballot_sync(0xffffffffu, known && o.small);
+            switched += __popc(__ballot_sync(0xffffffffu, known && o.switched));
             const bool major_small = 2 * __popc(sm) >= __popc(am);
-            const bool defer = queues && act && o.small != major_small;
+            const bool defer = queues && known && o.small != major_small;
             const unsigned dm = __ballot_sync(0xffffffffu, defer);
             if (dm) {
                 // the deferred lanes' mode is the other one: small when the majority is large
@@ -582,7 +639,16 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
             }
             act = act && !defer;
         }
-        if (act) {
+        if (kLinksInt) {
+            bool div = false;
+            LinkPose p;
+            __syncthreads();
+            if (act && !plain) plain = !link_pose_int(ip, sims[e.x], e.y, o, &p);
+            __syncthreads();
+            if (act && !plain) plain = !link_forces_int(ip, sims[e.x], e.y, ctl[e.x].dt, p, &div);
+            if (act && plain) div = link_plain(sims[e.x], e.y, ctl[e.x].dt);
+            if (div) ctl[e.x].diverged = 1;
+        } else if (act) {
             Ctl& c = ctl[e.x];
             bool div = false;
             link_finish(sims[e.x], e.y, c.dt, o, &div);

@@ -2,6 +2,7 @@
 // become single FP64 FMA instructions (fewer instructions on the FP64 pipe,
 // results within the parity tolerance instead of bit-faithful).
 #define GVX_KNS kfast
+#define GVX_CONTRACT 1   // products stay on the FP64 pipe, where they contract with their sums
 #include "kernelset.h"
 #include "kernels.cuh"
 

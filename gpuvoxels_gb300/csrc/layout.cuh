@@ -32,6 +32,7 @@ constexpr uint8_t LF_WIDE2 = 8;           // last step: angle2's rotation vector
 constexpr uint8_t LF_ACOS1 = 16;          // last step: angle1's rotation vector took the acos branch
 constexpr uint8_t LF_GONE = 32;           // VX3: detached (failed) or removed with a voxel: no longer updated
 constexpr uint8_t LF_REMOVED = 64;        // VX3: removed with a voxel (left out of the history's link records)
+constexpr uint8_t LF_PLAIN = 128;         // last step: taken by the plain form of the update (not shown to callers)
 constexpr uint32_t VF_FLOORC = 1u << 10;  // last step: the voxel touched the floor
 constexpr uint32_t VF_REMOVED = 1u << 11; // VX3: removed from the simulation (frozen, no links, no contacts)
 constexpr uint32_t VF_TGTHIT = 1u << 12;  // VX3: this step's contacts include a target voxel (non-target voxel)
