@@ -1466,6 +1466,23 @@ public:
         return std::max(1, std::min(n_items, sm_count_ * per_sm));
     }
 
+    // Launch shape of k_links (which = 0) and k_voxels (1) for `elems` elements in warp chunks of
+    // `claim`.  A batch with chunks for every resident warp takes the persistent grid of `block`
+    // threads.  A smaller one gives each SM the same number of warps, in as few blocks as hold
+    // them: the SM's one FP64 unit is what its warps share, so eight warps of one block cost a
+    // small batch eight warps' time while other SMs idle (a 10^3 creature: k_links on 4 blocks
+    // of 8 warps 40-44 us, on 31 blocks of one warp 34-37 us; the serving stream 41.3 -> 35.8 ms).
+    struct Shape { int grid, block; };
+    Shape grid_shape(size_t elems, int block, int claim, int which) {
+        block = std::min(block, ks_.max_block);
+        const size_t chunks = std::max<size_t>(1, (elems + claim - 1) / claim), sms = (size_t)sm_count_;
+        const size_t per_sm = (size_t)ks_.resident_blocks(which, block), most = (size_t)block / 32;   // blocks an SM, warps a block
+        const size_t want = (chunks + sms - 1) / sms;                                                // warps an SM
+        if (want >= most * per_sm) return {(int)(sms * per_sm), block};
+        const size_t blocks = (want + most - 1) / most, warps = (want + blocks - 1) / blocks;
+        return {(int)((chunks + warps - 1) / warps), (int)(32 * warps)};
+    }
+
     // One step of the batch; returns the number of kernels it launched.
     int launch_step(cudaStream_t st, bool prof) {
         int launched = 3 + (any_collide_ ? 1 : 0) + (any_watch_ ? 3 : 0) + (any_signals_ ? 1 : 0) + (n_attach_ ? 1 : 0);
@@ -1488,15 +1505,9 @@ public:
         }
         bin_phase_++;
         if (prof) cudaEventRecord(evk_[0], st);
-        // persistent grids, but no more blocks than the batch has block-sized pieces: every warp
-        // of a block claims at least one chunk, and idle claims cost atomics in small batches
-        const int bl = std::min(block_links_, ks_.max_block), bv = std::min(block_voxels_, ks_.max_block);
-        auto grid_chunks = [&](size_t elems, int block, int which) {
-            const size_t full = (size_t)sm_count_ * ks_.resident_blocks(which, block);
-            return (int)std::max<size_t>(1, std::min(full, (elems + block - 1) / block));
-        };
-        ks_.links(grid_chunks(batch_links_, bl, 0), bl, st, d_sims_, d_ctl_, d_link_perm_, d_link_total_,
-                  (int)cap_perm_, cap_slots_, d_tickets_, claim_links_);
+        // persistent grids; a batch that does not fill them is spread evenly over the SMs
+        const Shape ls = grid_shape(batch_links_, block_links_, claim_links_, 0), vs = grid_shape(batch_voxels_, block_voxels_, claim_voxels_, 1);
+        ks_.links(ls.grid, ls.block, st, d_sims_, d_ctl_, d_link_perm_, d_link_total_, (int)cap_perm_, cap_slots_, d_tickets_, claim_links_);
         if (prof) cudaEventRecord(evk_[1], st);
         // the watch-list passes: a persistent grid of 256-thread blocks over the listed items' work units
         if (any_watch_) ks_.watch(4 * sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_, d_stale_items_, d_tickets_, d_batch_slots_,
@@ -1505,8 +1516,7 @@ public:
         if (n_attach_) ks_.attach(st, d_sims_, d_ctl_, d_attach_slots_, n_attach_);
         if (prof) cudaEventRecord(evk_[2], st);
         if (prof) cudaEventRecord(evk_[3], st);
-        ks_.voxels(grid_chunks(batch_voxels_, bv, 1), bv, st, d_sims_, d_ctl_, d_vox_perm_, d_vox_total_,
-                   (int)cap_vperm_, cap_slots_, d_tickets_, claim_voxels_);
+        ks_.voxels(vs.grid, vs.block, st, d_sims_, d_ctl_, d_vox_perm_, d_vox_total_, (int)cap_vperm_, cap_slots_, d_tickets_, claim_voxels_);
         if (prof) cudaEventRecord(evk_[4], st);
         ks_.sim_end(st, d_sims_, d_ctl_, d_batch_slots_, n_batch_, d_tickets_, d_stale_items_);
         if (any_signals_) ks_.signals(grid_for(n_vox_items_, 256), 256, st, d_sims_, d_ctl_, vi, n_vox_items_, d_tickets_);
