@@ -2056,7 +2056,7 @@ public:
         for (int i = 0; i < nv; i++) {
             if (d13) for (int k = 0; k < 13; k++) d13[13 * (size_t)i + k] = buf[(size_t)k * nv + i];
             if (f4) { f4[4 * (size_t)i] = tb[i]; for (int k = 0; k < 3; k++) f4[4 * (size_t)i + 1 + k] = ps[(size_t)k * nv + i]; }
-            if (flags) flags[i] = (int32_t)fl[i];
+            if (flags) flags[i] = (int32_t)(fl[i] & ~dev::VF_PLAIN);
         }
         return 0;
     }

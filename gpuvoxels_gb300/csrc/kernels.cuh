@@ -1188,9 +1188,63 @@ __device__ void frozen_voxel(const Sim& S, int v, uint32_t fl, const VMat& m, co
     if ((flags & SF_COLLIDE) && !(fl & (VF_INTERIOR | VF_REMOVED))) hash_insert(S, v, pos, S.temp[v], hash_next_table);
 }
 
+// The end of a voxel's step, after its state is stored: the Poisson strain the next step's links
+// will read, its signals, the next step's temperature, the contact hash and the watch-list check.
+__device__ __forceinline__ void voxel_after(const Sim& S, int v, const VMat& m, uint32_t fl, const Ext* e, const d3& pos, float temp,
+                                            const StepTimes& st, int flags, int* hash_next_table, int* watch_moved) {
+    const int nv = S.nv;
+    const bool fixed_all = e && (e->dof & 0x3F) == 0x3F;
+    // CVX_Voxel::strain(true) for the next step (fully fixed voxels keep their cached value)
+    if (!fixed_all && m.nu != 0.0f) {
+        float s[3] = {0, 0, 0};
+        int nb[3] = {0, 0, 0};
+#pragma unroll
+        for (int d = 0; d < 6; d++)
+            if (fl & (1u << d)) { s[d >> 1] += S.ss[d * nv + v]; nb[d >> 1]++; }
+        bool ten[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            if (nb[i] == 2) s[i] *= 0.5f;
+            ten[i] = (nb[i] == 2) || (e && nb[i] == 1 && ((e->dof & (1 << i)) || e->f[i] != 0));
+        }
+        if (!(ten[0] && ten[1] && ten[2])) {
+            float add = 0;
+            for (int i = 0; i < 3; i++) if (ten[i]) add += s[i];
+            const float value = poisson_power(m, 1.0f + add) - 1.0f;
+            for (int i = 0; i < 3; i++) if (!ten[i]) s[i] = value;
+        }
+        S.ps[v] = s[0]; S.ps[nv + v] = s[1]; S.ps[2 * nv + v] = s[2];
+    }
+    // VX3 signals: the voxel's own signal work at the end of its step (a voxel fixed in all
+    // degrees of freedom returns from VX3_Voxel::timeStep before it, VX3_Voxel.cu:166-173)
+    if (flags & SF_SIGNALS) {
+        if (!fixed_all) sig_own_step(S, v, m, st.t_now);
+        else S.sig[SG_OUT * (size_t)nv + v] = 0;
+    }
+    // actuation temperature for the next step
+    float temp_next = temp;
+    // (VX3: no update before the material's TurnOnThermalExpansionAfterThisManySeconds)
+    if ((flags & SF_VARY) && !fp64i::gt(m.thermalOn, st.t_next)) {
+        const float two_pi = 2 * 3.1415926f;
+        double T = S.temp_amp * sin((double)two_pi * (st.t_cycles + __ldg(S.phase + v)));
+        if (!(flags & SF_EXPAND) && fp64i::gt0(T)) T = 0;
+        temp_next = d2f(T);
+        S.temp[v] = temp_next;
+    }
+    // insert into the table the next step's contact pass reads
+    if ((flags & SF_COLLIDE) && !(fl & VF_INTERIOR)) hash_insert(S, v, pos, temp_next, hash_next_table);
+    // watch lists: a surface voxel further than the re-check distance from where the last
+    // regeneration saw it makes the next step regenerate (CVoxelyze::updateCollisions,
+    // Voxelyze.cpp:689-697: (pos - lastColWatchPosition).Length2() > recalcDist*recalcDist)
+    if (watch_moved && !(fl & VF_INTERIOR)) {
+        const float4 wp = S.watch[v];
+        const double dx = pos.x - (double)wp.x, dy = pos.y - (double)wp.y, dz = pos.z - (double)wp.z;
+        if (dx * dx + dy * dy + dz * dz > (double)S.recalc2) *watch_moved = 1;
+    }
+}
+
 __device__ __forceinline__ void voxel_update(const Sim& S, int v, float dt, const StepTimes& st, int flags, double* com4, int* hash_next_table,
                                              int* watch_moved = nullptr) {
-    const double t_cycles = st.t_cycles;
     const int nv = S.nv;
     const VMat& m = S.vm[__ldg(S.vmat + v)];
     uint32_t fl = S.vfl[v];
@@ -1350,53 +1404,19 @@ __device__ __forceinline__ void voxel_update(const Sim& S, int v, float dt, cons
         const double w = m.mass;
         com4[0] += pos.x * w; com4[1] += pos.y * w; com4[2] += pos.z * w; com4[3] += w;
     }
-    // CVX_Voxel::strain(true) for the next step (fully fixed voxels keep their cached value)
-    if (!fixed_all && m.nu != 0.0f) {
-        float s[3] = {0, 0, 0};
-        int nb[3] = {0, 0, 0};
-#pragma unroll
-        for (int d = 0; d < 6; d++)
-            if (fl & (1u << d)) { s[d >> 1] += S.ss[d * nv + v]; nb[d >> 1]++; }
-        bool ten[3];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            if (nb[i] == 2) s[i] *= 0.5f;
-            ten[i] = (nb[i] == 2) || (e && nb[i] == 1 && ((e->dof & (1 << i)) || e->f[i] != 0));
-        }
-        if (!(ten[0] && ten[1] && ten[2])) {
-            float add = 0;
-            for (int i = 0; i < 3; i++) if (ten[i]) add += s[i];
-            const float value = poisson_power(m, 1.0f + add) - 1.0f;
-            for (int i = 0; i < 3; i++) if (!ten[i]) s[i] = value;
-        }
-        S.ps[v] = s[0]; S.ps[nv + v] = s[1]; S.ps[2 * nv + v] = s[2];
-    }
-    // VX3 signals: the voxel's own signal work at the end of its step (a voxel fixed in all
-    // degrees of freedom returns from VX3_Voxel::timeStep before it, VX3_Voxel.cu:166-173)
-    if (flags & SF_SIGNALS) {
-        if (!fixed_all) sig_own_step(S, v, m, st.t_now);
-        else S.sig[SG_OUT * (size_t)nv + v] = 0;
-    }
-    // actuation temperature for the next step
-    float temp_next = temp;
-    // (VX3: no update before the material's TurnOnThermalExpansionAfterThisManySeconds)
-    if ((flags & SF_VARY) && !fp64i::gt(m.thermalOn, st.t_next)) {
-        const float two_pi = 2 * 3.1415926f;
-        double T = S.temp_amp * sin((double)two_pi * (t_cycles + __ldg(S.phase + v)));
-        if (!(flags & SF_EXPAND) && fp64i::gt0(T)) T = 0;
-        temp_next = d2f(T);
-        S.temp[v] = temp_next;
-    }
-    // insert into the table the next step's contact pass reads
-    if ((flags & SF_COLLIDE) && !(fl & VF_INTERIOR)) hash_insert(S, v, pos, temp_next, hash_next_table);
-    // watch lists: a surface voxel further than the re-check distance from where the last
-    // regeneration saw it makes the next step regenerate (CVoxelyze::updateCollisions,
-    // Voxelyze.cpp:689-697: (pos - lastColWatchPosition).Length2() > recalcDist*recalcDist)
-    if (watch_moved && !(fl & VF_INTERIOR)) {
-        const float4 wp = S.watch[v];
-        const double dx = pos.x - (double)wp.x, dy = pos.y - (double)wp.y, dz = pos.z - (double)wp.z;
-        if (dx * dx + dy * dy + dz * dz > (double)S.recalc2) *watch_moved = 1;
-    }
+    voxel_after(S, v, m, fl, e, pos, temp, st, flags, hash_next_table, watch_moved);
+}
+
+}  // namespace GVX_KNS
+}  // namespace gvx
+#include "voxels_int.cuh"
+namespace gvx {
+namespace GVX_KNS {
+
+// The plain form of a voxel's step (see link_plain).
+__device__ __noinline__ void voxel_plain(const Sim& S, int v, float dt, const StepTimes& st, int* hash_next_table, int* watch_moved) {
+    voxel_update(S, v, dt, st, S.flags, nullptr, hash_next_table, watch_moved);
+    S.vfl[v] |= VF_PLAIN;
 }
 
 __device__ __forceinline__ double block_sum(double x, double* red) {
@@ -1534,25 +1554,39 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
     }
     const int n = min(*total, cap);
     const int lane = threadIdx.x & 31;
+    int k = 0, k1 = 0;           // the claimed chunk: next round's first voxel, its end
+    bool more = true;            // chunks may remain
     for (;;) {
-        int chunk = 0;
-        if (lane == 0) chunk = atomicAdd(&tickets[2], 1);
-        chunk = __shfl_sync(0xffffffffu, chunk, 0);
-        const int k0 = chunk * claim;
-        if (k0 >= n) break;
-        const int k1 = min(n, k0 + claim);
-        for (int k = k0 + lane; k < k1; k += 32) {
-            const int2 e = __ldg(perm + k);
-            if ((unsigned)e.x >= (unsigned)n_slots) continue;   // never: the grouping lists running slots
-            const Ctl& c = ctl[e.x];
-            const float dt = c.dt;
-            if (c.status == 1 && !c.diverged && dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv) {
-                const Sim& S = sims[e.x];
-                StepTimes st;
-                st.t_now = c.t; st.t_next = c.t + dt; st.t_cycles = c.t_cycles; st.angle = c.recent_angle;
-                st.closeness = c.closeness; st.close_pairs = c.num_close_pairs; st.hits = c.hit_count;
-                int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
-                voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr);
+        if (k >= k1 && more) {
+            int chunk = 0;
+            if (lane == 0) chunk = atomicAdd(&tickets[2], 1);
+            chunk = __shfl_sync(0xffffffffu, chunk, 0);
+            k = chunk * claim;
+            k1 = min(n, k + claim);
+            if (k >= n) more = false;
+        }
+        // a block's warps keep step through the integer-pipe form (see k_links)
+        if (kLinksInt ? !__syncthreads_or(k < k1) : k >= k1) break;
+        int2 e = make_int2(-1, -1);
+        if (k + lane < k1) e = __ldg(perm + k + lane);
+        k += 32;
+        if ((unsigned)e.x >= (unsigned)n_slots) continue;   // none, or never: the grouping lists running slots
+        const Ctl& c = ctl[e.x];
+        const float dt = c.dt;
+        if (c.status == 1 && !c.diverged && dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv) {
+            const Sim& S = sims[e.x];
+            StepTimes st;
+            st.t_now = c.t; st.t_next = c.t + dt; st.t_cycles = c.t_cycles; st.angle = c.recent_angle;
+            st.closeness = c.closeness; st.close_pairs = c.num_close_pairs; st.hits = c.hit_count;
+            int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
+            int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
+            if (kLinksInt) {
+                const uint32_t fl = S.vfl[e.y];
+                bool plain = (S.flags & SF_VOXEL_EXTRAS) || (fl & VF_EXT) || ((fl & VF_PLAIN) && !plain_retry(c.steps));
+                if (!plain) plain = !voxel_update_int(S, e.y, fl, dt, st, S.flags, hnext, moved);
+                if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
+            } else {
+                voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, moved);
             }
         }
     }

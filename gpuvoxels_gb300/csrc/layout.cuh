@@ -38,6 +38,7 @@ constexpr uint32_t VF_REMOVED = 1u << 11; // VX3: removed from the simulation (f
 constexpr uint32_t VF_TGTHIT = 1u << 12;  // VX3: this step's contacts include a target voxel (non-target voxel)
 constexpr uint32_t VF_ATTACH = 1u << 13;  // VX3: enableAttach (every attach condition holds at the voxel)
 constexpr uint32_t VF_WROT = 1u << 14;    // last step: the orientation update took the sin/cos branch (grouping key only)
+constexpr uint32_t VF_PLAIN = 1u << 15;   // last step: taken by the plain form of the update (not shown to callers)
 
 // sim flag bits
 constexpr int SF_FLOOR = 1, SF_COLLIDE = 2, SF_VARY = 4, SF_EXPAND = 8;

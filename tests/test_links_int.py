@@ -1,4 +1,4 @@
-"""The integer-pipe form of the link update: its exact operations against IEEE arithmetic (host and
+"""The integer-pipe forms of the link and voxel updates: their exact operations against IEEE arithmetic (host and
 device), and whole bodies on it and on the plain form it falls back to against the CPU oracle."""
 import os
 import shutil
@@ -39,6 +39,10 @@ BODIES = [("beam_1x1x9", (1, 1, 9), [MAT], True, {}), ("one_link", (2, 1, 1), [M
           ("undamped", (4, 4, 4), [MAT], False, dict(damping=(0.0, 0.8, 0.01))),
           ("no_poisson", (4, 3, 5), [dict(MAT, nu=0.0)], False, {}),
           ("two_stiffnesses", (7, 6, 5), [MAT, dict(MAT, E=2e5, cte=0.0)], False, {}),
+          ("no_floor", (4, 4, 3), [MAT], False, dict(floor=False)),
+          ("sliding", (6, 6, 2), [dict(MAT, mus=0.3, muk=0.2)], False, dict(temp_period=0.004)),
+          ("frictionless", (5, 5, 2), [dict(MAT, mus=0.0, muk=0.0)], False, dict(temp_period=0.004)),
+          ("undamped_voxels", (4, 4, 4), [MAT], False, dict(damping=(1.0, 0.0, 0.0))),
           ("large_angles", (9, 3, 3), [dict(MAT, E=1e5, cte=0.02)], False, dict(temp_period=0.02))]
 
 
@@ -65,4 +69,6 @@ def test_links_against_the_oracle(name, side, mats, same, kw, steps):
     w = o.voxel_state()
     assert np.abs(v["pos"] - w["pos"]).max() <= 1e-6 * 0.01
     assert np.abs(v["orient"] - w["orient"]).max() <= 1e-6
+    static = (v["flags"] >> 6) & 1
+    assert np.array_equal(static, (w["flags"] & 8) >> 3) and v["flags"].max() < 1 << 15
     assert l["flags"].max() < 128 and np.isfinite(l["pos2"]).all()
