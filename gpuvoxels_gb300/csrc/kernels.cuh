@@ -5,9 +5,18 @@
 // simulations share one launch with no per-simulation launch overhead.
 #pragma once
 #include "physics.cuh"
+#include "trig_int.cuh"
 
 namespace gvx {
 namespace GVX_KNS {
+
+// Whether links and voxels take the integer-pipe forms (links_int.cuh, voxels_int.cuh): the exact
+// build does; the FMA build's products contract with their sums on the FP64 pipe.
+#ifdef GVX_CONTRACT
+constexpr bool kIntPipes = false;
+#else
+constexpr bool kIntPipes = true;
+#endif
 
 constexpr float HB_TURN = 1.2f * 0.05f;   // HYSTERESIS_FACTOR*SA_BOND_BEND_RAD (types.h:57-58)
 constexpr float HB_EXT = 1.2f * 0.50f;    // HYSTERESIS_FACTOR*SA_BOND_EXT_PERC (types.h:57-59)
@@ -267,14 +276,6 @@ __device__ __forceinline__ void link_finish(const Sim& S, int l, float dt, const
 #include "links_int.cuh"
 namespace gvx {
 namespace GVX_KNS {
-
-// Whether links take the integer-pipe form (links_int.cuh): the exact build does; the FMA build's
-// products contract with their sums on the FP64 pipe.
-#ifdef GVX_CONTRACT
-constexpr bool kLinksInt = false;
-#else
-constexpr bool kLinksInt = true;
-#endif
 
 // The plain form of a whole link update, for a link that the integer-pipe form left (out of line:
 // rare once a body moves).  Sets LF_PLAIN, which keeps the link on this form until plain_retry, so
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
         }
         // the integer-pipe form is long straight-line code: a block's warps keep step through it
         // (here, and between its three parts below), so that one of them fetches it for all
-        if (kLinksInt ? !__syncthreads_or(src != 2) : src == 2) break;
+        if (kIntPipes ? !__syncthreads_or(src != 2) : src == 2) break;
         int2 e = make_int2(-1, -1);
         if (src == 2) {
         } else if (src < 0) {
@@ -608,7 +609,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
         LinkOrient o;
         IntPipes ip;
         bool plain = false;      // this link takes the plain form (and is not deferred)
-        if (kLinksInt) {
+        if (kIntPipes) {
             if (act) {
                 const Sim& S = sims[e.x];
                 const uint8_t fl = S.lfl[e.y];
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
             }
             act = act && !defer;
         }
-        if (kLinksInt) {
+        if (kIntPipes) {
             bool div = false;
             LinkPose p;
             __syncthreads();
@@ -1226,9 +1227,12 @@ __device__ __forceinline__ void voxel_after(const Sim& S, int v, const VMat& m, 
     // (VX3: no update before the material's TurnOnThermalExpansionAfterThisManySeconds)
     if ((flags & SF_VARY) && !fp64i::gt(m.thermalOn, st.t_next)) {
         const float two_pi = 2 * 3.1415926f;
-        double T = S.temp_amp * sin((double)two_pi * (st.t_cycles + __ldg(S.phase + v)));
-        if (!(flags & SF_EXPAND) && fp64i::gt0(T)) T = 0;
-        temp_next = d2f(T);
+        const double turn = (double)two_pi * (st.t_cycles + __ldg(S.phase + v));
+        const bool contract_only = !(flags & SF_EXPAND);
+        uint32_t rare = kIntPipes ? 0u : fp64i::kOutOfBand;
+        if (kIntPipes) temp_next = fp64i::sin_times_band(S.temp_amp, turn, rare);
+        if (rare & fp64i::kOutOfBand) temp_next = d2f(S.temp_amp * sin(turn));
+        if (contract_only && temp_next > 0) temp_next = 0;
         S.temp[v] = temp_next;
     }
     // insert into the table the next step's contact pass reads
@@ -1566,7 +1570,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
             if (k >= n) more = false;
         }
         // a block's warps keep step through the integer-pipe form (see k_links)
-        if (kLinksInt ? !__syncthreads_or(k < k1) : k >= k1) break;
+        if (kIntPipes ? !__syncthreads_or(k < k1) : k >= k1) break;
         int2 e = make_int2(-1, -1);
         if (k + lane < k1) e = __ldg(perm + k + lane);
         k += 32;
@@ -1580,7 +1584,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
             st.closeness = c.closeness; st.close_pairs = c.num_close_pairs; st.hits = c.hit_count;
             int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
             int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
-            if (kLinksInt) {
+            if (kIntPipes) {
                 const uint32_t fl = S.vfl[e.y];
                 bool plain = (S.flags & SF_VOXEL_EXTRAS) || (fl & VF_EXT) || ((fl & VF_PLAIN) && !plain_retry(c.steps));
                 if (!plain) plain = !voxel_update_int(S, e.y, fl, dt, st, S.flags, hnext, moved);
