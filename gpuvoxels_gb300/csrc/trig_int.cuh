@@ -28,7 +28,7 @@ GVX_FP64I int clz64(uint64_t x) {
 // V * 2^e for V in [2^62, 2^64), rounded to 53 bits; e such that the result is normal.
 GVX_FP64I double round64(uint64_t V, int e) {
     const int s = 10 + (int)(V >> 63);
-    const uint64_t r = (V + (1ull << (s - 1))) >> s;   // 2^52..2^53
+    const uint64_t r = (V >> s) + ((V >> (s - 1)) & 1u);   // 2^52..2^53 (V + half could pass 2^64)
     return from_bits(r + ((uint64_t)(uint32_t)(e + s + 1023 + 51) << 52));
 }
 // sin(y) for |y| in [2^-10, 2^20): y/(2 pi) to 2^-64 of a turn, folded into a quarter turn R, and

@@ -72,7 +72,9 @@ GVX_FP64I int one_case(uint64_t i, uint32_t* in_band) {
     q = f2d_band(f, r);
     check(5, bits(q) == bits((double)f));
     const double amp = ldexp(1.0 + (double)(t & 0xFFFFF) * 0x1p-20, (int)(t % 17) - 8) * ((t >> 20) & 1 ? 1.0 : -1.0);
-    const double turn = from_bits(with_exponent(a, 1023 - 14 + (uint32_t)((t >> 21) % 36)));
+    double turn = from_bits(with_exponent(a, 1023 - 14 + (uint32_t)((t >> 21) % 36)));
+    if (mode & 4)   // within 2^-20..2^-50 of a multiple of pi/2: results next to 0 and to +-1
+        turn = (double)(int)((t >> 26) % 4096 + 1) * 1.5707963267948966 * (1.0 + ldexp((double)(int)(t % 7) - 3.0, -20 - (int)((t >> 40) % 34)));
     f = sin_times_band(amp, turn, r);
     check(6, fbits(f) == fbits((float)(amp * sin(turn))));
     // an operand that is zero, subnormal, infinite or NaN is always found
