@@ -1592,17 +1592,13 @@ public:
         return 0;
     }
 
-    // Runs until every listed simulation has left the RUNNING state.
-    int drive(const std::vector<SimRec*>& rs, int mode, std::string* err) {
+    // Runs until every listed simulation has left the RUNNING state.  cs: the control blocks of the slots
+    // from slo on as they were before (read by the caller); on return as they are now.
+    int drive(const std::vector<SimRec*>& rs, int mode, std::string* err, std::vector<dev::Ctl>& cs, int slo) {
         int64_t vsteps_before = 0;
         std::vector<int64_t> steps0(rs.size());
-        int slo = INT32_MAX, shi = -1;
-        for (auto* r : rs) { slo = std::min(slo, r->slot); shi = std::max(shi, r->slot); }
-        std::vector<dev::Ctl> cs;
-        if (!rs.empty()) {
-            if (int e = read_ctls(slo, shi, &cs, err)) return e;
-            for (size_t i = 0; i < rs.size(); i++) steps0[i] = cs[(size_t)(rs[i]->slot - slo)].steps;
-        }
+        const int shi = slo + (int)cs.size() - 1;
+        for (size_t i = 0; i < rs.size(); i++) steps0[i] = cs[(size_t)(rs[i]->slot - slo)].steps;
         timing_.launches = 0;
         double w0 = now_s();
         CK(cudaEventRecord(ev0_, stream_));
@@ -1685,7 +1681,11 @@ public:
             }
         }
         CK(cudaEventRecord(ev1_, stream_));
-        CK(cudaEventSynchronize(ev1_));
+        if (!rs.empty()) {
+            if (int e = read_ctls(slo, shi, &cs, err)) return e;   // waits for the steps as well
+        } else {
+            CK(cudaEventSynchronize(ev1_));
+        }
         float ms = 0;
         cudaEventElapsedTime(&ms, ev0_, ev1_);
         timing_.device_ms = ms;
@@ -1697,13 +1697,10 @@ public:
             cudaEventElapsedTime(&c, evk_[3], evk_[4]);   // k_voxels
             timing_.link_kernel_ms = a; timing_.contact_kernel_ms = b; timing_.voxel_kernel_ms = c;
         }
-        if (!rs.empty()) {
-            if (int e = read_ctls(slo, shi, &cs, err)) return e;
-            for (size_t i = 0; i < rs.size(); i++) {
-                const dev::Ctl& c = cs[(size_t)(rs[i]->slot - slo)];
-                rs[i]->status = c.status;
-                vsteps_before += (c.steps - steps0[i]) * rs[i]->w.nv;
-            }
+        for (size_t i = 0; i < rs.size(); i++) {
+            const dev::Ctl& c = cs[(size_t)(rs[i]->slot - slo)];
+            rs[i]->status = c.status;
+            vsteps_before += (c.steps - steps0[i]) * rs[i]->w.nv;
         }
         timing_.voxel_steps = vsteps_before;
         return 0;
@@ -1772,12 +1769,15 @@ public:
         if (int e = set_running(slots, targets, err, 1)) return e;
         tc.mark("step: read/set control");
         exact_steps_ = steps;
-        int e = drive(act, mode, err);
+        int e = drive(act, mode, err, cs, lo);
         tc.mark("step: drive");
         exact_steps_ = -1;
         if (int e2 = end_fixed_steps(slots, err)) return e2;
-        if (int e2 = read_ctls(lo, hi, &cs, err)) return e2;
-        for (auto* r : act) r->status = cs[(size_t)(r->slot - lo)].status;
+        if (e) return e;
+        for (auto* r : act) {   // what end_fixed_steps leaves on the device
+            const int st = cs[(size_t)(r->slot - lo)].status;
+            r->status = st == SIM_DONE ? SIM_IDLE : st;
+        }
         tc.mark("step: end");
         return e;
     }
@@ -1808,10 +1808,10 @@ public:
         }
         if (act.empty()) return 0;
         if (int e = set_running(slots, targets, err)) return e;
-        int e = drive(act, mode, err);
+        int e = drive(act, mode, err, cs, lo);
         if (e) return e;
-        for (auto* r : act) finish(r, r->status, err);
-        return 0;
+        for (auto* r : act) r->retired = false;
+        return finish_many(act, err);
     }
 
     int com(SimRec* r, double* out, std::string* err) {
@@ -1829,6 +1829,25 @@ public:
     int finish(SimRec* r, int status, std::string* err) {
         dev::Ctl c;
         if (int e = read_ctl(r->slot, &c, err)) return e;
+        double com3[3];
+        if (int e = com(r, com3, err)) return e;
+        const size_t nv = r->w.nv;
+        std::vector<double> p(3 * nv), ip;
+        CK(copy_async(p.data(), r->dsim.px, 8 * nv, cudaMemcpyDeviceToHost, stream_));
+        CK(copy_async(p.data() + nv, r->dsim.py, 8 * nv, cudaMemcpyDeviceToHost, stream_));
+        CK(copy_async(p.data() + 2 * nv, r->dsim.pz, 8 * nv, cudaMemcpyDeviceToHost, stream_));
+        if (c.reinit_done) {
+            ip.resize(3 * nv);
+            CK(copy_async(ip.data(), r->dsim.init_pos, 8 * 3 * nv, cudaMemcpyDeviceToHost, stream_));
+        }
+        CK(cudaStreamSynchronize(stream_));
+        finish_from(r, status, c, com3, p.data(), ip.empty() ? nullptr : ip.data());
+        return 0;
+    }
+
+    // The result of a simulation from its control block, final centre of mass and positions (x, y and z
+    // blocks); ip: its initial positions where the secondary experiment reset them, else null.
+    void finish_from(SimRec* r, int status, const dev::Ctl& c, const double* com3, const double* p, const double* ip) {
         SimResult& R = r->result;
         R = SimResult{};
         R.id = r->id;
@@ -1840,7 +1859,7 @@ public:
         R.vox_size = r->w.desc.vox_size;
         // initial centre of mass: the host's, or the one the secondary experiment reset it to
         for (int k = 0; k < 3; k++) R.initial_com[k] = c.reinit_done ? c.init_com[k] : r->init_com[k];
-        if (int e = com(r, R.current_com, err)) return e;
+        for (int k = 0; k < 3; k++) R.current_com[k] = com3[k];
         R.num_close_pairs = c.num_close_pairs;
         MathVars mv{R.current_com[0] - R.initial_com[0], R.current_com[1] - R.initial_com[1], R.current_com[2] - R.initial_com[2],
                     (double)c.hit_count, c.t, c.recent_angle, c.closeness, c.num_close_pairs, r->w.nv};
@@ -1848,29 +1867,21 @@ public:
         // total distance travelled by measured voxels from their initial positions
         // (VX3_SimulationManager.cu:442-452)
         const size_t nv = r->w.nv;
-        std::vector<double> p(3 * nv), ip;
-        CK(copy_async(p.data(), r->dsim.px, 8 * nv, cudaMemcpyDeviceToHost, stream_));
-        CK(copy_async(p.data() + nv, r->dsim.py, 8 * nv, cudaMemcpyDeviceToHost, stream_));
-        CK(copy_async(p.data() + 2 * nv, r->dsim.pz, 8 * nv, cudaMemcpyDeviceToHost, stream_));
-        if (c.reinit_done) {
-            ip.resize(3 * nv);
-            CK(copy_async(ip.data(), r->dsim.init_pos, 8 * 3 * nv, cudaMemcpyDeviceToHost, stream_));
-        }
-        CK(cudaStreamSynchronize(stream_));
         double tot = 0;
         for (size_t i = 0; i < nv; i++) {
             if (!r->w.vmats[r->w.desc.voxels[4 * i + 3]].is_measured) continue;
             double nom = r->w.vmats[r->w.desc.voxels[4 * i + 3]].nom;
-            const double ix = ip.empty() ? r->w.desc.voxels[4 * i] * nom : ip[i];
-            const double iy = ip.empty() ? r->w.desc.voxels[4 * i + 1] * nom : ip[nv + i];
-            const double iz = ip.empty() ? r->w.desc.voxels[4 * i + 2] * nom : ip[2 * nv + i];
+            const double ix = !ip ? r->w.desc.voxels[4 * i] * nom : ip[i];
+            const double iy = !ip ? r->w.desc.voxels[4 * i + 1] * nom : ip[nv + i];
+            const double iz = !ip ? r->w.desc.voxels[4 * i + 2] * nom : ip[2 * nv + i];
             double dx = p[i] - ix, dy = p[nv + i] - iy, dz = p[2 * nv + i] - iz;
             tot += sqrt(dx * dx + dy * dy + dz * dz);
         }
         R.total_distance = tot;
         if (r->w.desc.save_all_positions) {   // kept for the report's pos and init_pos fields
-            r->final_pos = std::move(p);
-            r->final_init_pos = std::move(ip);
+            r->final_pos.assign(p, p + 3 * nv);
+            if (ip) r->final_init_pos.assign(ip, ip + 3 * nv);
+            else r->final_init_pos.clear();
         }
         R.submit_s = r->submit_s;
         R.start_s = r->start_s;
@@ -1878,7 +1889,74 @@ public:
         R.finish_s = r->finish_s;
         r->status = R.status;
         r->retired = true;
+    }
+
+    // The results of several simulations with one kernel, one copy and one wait for all of them, and
+    // their sums on host threads (one by one each took four waits and three copies, about 70 us a
+    // simulation).  Simulations that reset their initial positions, and lists too large for the pinned
+    // buffer or the arena's free space, are finished one by one.
+    int finish_many(const std::vector<SimRec*>& rs, std::string* err) {
+        std::vector<SimRec*> many;
+        std::vector<dev::Ctl> cs;
+        int lo = INT32_MAX, hi = -1;
+        for (auto* r : rs) { lo = std::min(lo, r->slot); hi = std::max(hi, r->slot); }
+        size_t voxels = 0;
+        if (rs.size() > 1) {
+            if (int e = read_ctls(lo, hi, &cs, err)) return e;
+            for (auto* r : rs)
+                if (!cs[(size_t)(r->slot - lo)].reinit_done) { many.push_back(r); voxels += r->w.nv; }
+        }
+        const size_t n = many.size(), b_com = 32 * n, b_pos = 24 * voxels, b_idx = 12 * n;
+        const size_t need = b_com + b_pos + b_idx;
+        size_t off = 0;
+        if (n < 2 || b_com + b_pos > kPinnedUploadMax || !arena_.alloc(need, &off)) many.clear();
+        if (!many.empty()) {
+            struct ArenaTemp {   // gives the region back on every way out
+                EngineImpl* e; size_t off, n;
+                ~ArenaTemp() { cudaStreamSynchronize(e->stream_); e->arena_.release(off, n); }
+            } temp{this, off, need};
+            if (int e = pinned(&rb_, b_idx, err)) return e;
+            std::vector<int64_t> at(n);
+            int64_t total = 0;
+            for (size_t k = 0; k < n; k++) { at[k] = total; total += many[k]->w.nv; }
+            memcpy(rb_.p, at.data(), 8 * n);
+            for (size_t k = 0; k < n; k++) ((int*)(rb_.p + 8 * n))[k] = many[k]->slot;
+            char* d = arena_base_ + off;
+            CK(copy_async(d + b_com + b_pos, rb_.p, b_idx, cudaMemcpyHostToDevice, stream_));
+            CK(cudaEventRecord(rb_.done, stream_));
+            const int64_t* d_at = (const int64_t*)(d + b_com + b_pos);
+            ks_.pack_results(stream_, d_sims_, (const int*)(d_at + n), d_at, (int)n, (double*)d, (double*)(d + b_com));
+            CK(cudaGetLastError());
+            if (int e = pinned(&gen_, b_com + b_pos, err)) return e;
+            CK(copy_async(gen_.p, d, b_com + b_pos, cudaMemcpyDeviceToHost, stream_));
+            CK(cudaEventRecord(gen_.done, stream_));
+            CK(cudaEventSynchronize(gen_.done));
+            std::atomic<size_t> next{0};
+            auto work = [&]() {
+                for (size_t k = next++; k < n; k = next++) {
+                    const double* c4 = (const double*)gen_.p + 4 * k;
+                    double com3[3] = {0, 0, 0};
+                    if (c4[3] != 0) for (int j = 0; j < 3; j++) com3[j] = c4[j] / c4[3];
+                    finish_from(many[k], many[k]->status, cs[(size_t)(many[k]->slot - lo)], com3, (const double*)(gen_.p + b_com) + 3 * at[k], nullptr);
+                }
+            };
+            run_threads(voxels >= kThreadedVoxels ? n : 1, work);
+        }
+        for (auto* r : rs)
+            if (!r->retired)
+                if (int e = finish(r, r->status, err)) return e;
         return 0;
+    }
+    static constexpr size_t kThreadedVoxels = 8192;   // the work on fewer costs less than starting threads (about 80 us)
+
+    // Runs `work` on up to `most` threads, this one among them.
+    template <typename F>
+    static void run_threads(size_t most, const F& work) {
+        const size_t nt = std::max<size_t>(1, std::min<size_t>(most, std::max(1u, std::thread::hardware_concurrency())));
+        std::vector<std::thread> pool;
+        for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
+        work();
+        for (auto& t : pool) t.join();
     }
 
     // ---------------------------------------------------------------- serving
@@ -2131,6 +2209,7 @@ public:
         std::vector<int> slots((size_t)n);
         std::vector<int64_t> offs((size_t)n);
         int64_t total = 0;
+        int largest = 0;
         for (int k = 0; k < n; k++) {
             SimRec* r = find(ids[k]);
             if (!r) { *err = "unknown simulation id"; return -6; }
@@ -2138,8 +2217,11 @@ public:
             slots[k] = r->slot;
             offs[k] = total;
             total += r->w.nv;
+            largest = std::max(largest, r->w.nv);
         }
         if (total == 0) return 0;
+        // two voxels a thread of the largest simulation, within eight blocks an SM for the whole list
+        const int gx = std::max(8, std::min((largest + 511) / 512, 8 * sm_count_ / std::min(n, sm_count_) + 8));
         const size_t b_pos = 24 * (size_t)total, b_q = 32 * (size_t)total, b_fl = (size_t)total;
         const size_t b_idx = 4 * (size_t)n + 8 * (size_t)n;
         const size_t need = b_pos + b_q + b_fl + 16 + b_idx + 16;
@@ -2179,7 +2261,7 @@ public:
         const int64_t* doff = (const int64_t*)(dg + o_idx);
         const int* dslot = (const int*)(dg + o_idx + 8 * (size_t)n);
         for (int k0 = 0; k0 < n; k0 += 65535)
-            ks_.gather(stream_, d_sims_, dslot + k0, doff + k0, std::min(65535, n - k0), dpos, dq, dfl);
+            ks_.gather(stream_, d_sims_, dslot + k0, doff + k0, std::min(65535, n - k0), gx, dpos, dq, dfl);
         CK(cudaGetLastError());
         const size_t b_all = b_pos + b_q + b_fl;
         if (b_all <= kPinnedUploadMax) {
@@ -2214,11 +2296,7 @@ public:
             auto work = [&]() {
                 for (size_t i = next++; i < pieces.size(); i = next++) memcpy(pieces[i].dst, pieces[i].src, pieces[i].n);
             };
-            const int nt = (int)std::max<size_t>(1, std::min<size_t>(pieces.size(), std::max(1u, std::thread::hardware_concurrency())));
-            std::vector<std::thread> pool;
-            for (int t = 1; t < nt; t++) pool.emplace_back(work);
-            work();
-            for (auto& t : pool) t.join();
+            run_threads((size_t)total >= kThreadedVoxels ? pieces.size() : 1, work);
             tg.mark("gather: host copies");
             return 0;
         }

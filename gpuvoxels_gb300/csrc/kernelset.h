@@ -34,7 +34,7 @@ struct KernelSet {
     void (*com)(cudaStream_t s, const dev::Sim* sims, int sim, double* out4);
     // Packs position, orientation and the reference-order flag byte of the voxels of
     // n simulations (slot[k], output offset off[k]) into pos3 / q4 / flags (one launch).
-    void (*gather)(cudaStream_t s, const dev::Sim* sims, const int* slot, const int64_t* off, int n, double* pos3, double* q4,
+    void (*gather)(cudaStream_t s, const dev::Sim* sims, const int* slot, const int64_t* off, int n, int gx, double* pos3, double* q4,
                    uint8_t* flags);
     // resident blocks per SM of k_links (0) or k_voxels (1) at a block size
     int (*resident_blocks)(int which, int block);
@@ -44,6 +44,8 @@ struct KernelSet {
     // slot list
     void (*watch)(int grid, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n_items,
                   const int* stale_items, const int* tickets, const int* slots, int n_sims);
+    // packs the centre-of-mass sums (4 each) and the positions (x, y, z blocks at 3*off[k]) of n simulations
+    void (*pack_results)(cudaStream_t s, const dev::Sim* sims, const int* slot, const int64_t* off, int n, double* com4, double* pos);
 };
 
 KernelSet kernelset_exact();   // every multiply and add rounded separately (the reference's CPU rounding)

@@ -1,0 +1,39 @@
+"""Results and poses of many simulations taken together equal those taken one by one."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _docs(sides):
+    from gpuvoxels_gb300 import synth
+    return [synth.random_creature(40 + i, (s, s + 1, max(1, s - 1)), 0.8, stop_time=1.0).vxa for i, s in enumerate(sides)]
+
+
+@pytest.mark.parametrize("sides", [[3], [1, 4], [2, 5, 7, 3, 6], [16, 20, 18, 5]], ids=["one", "two", "five", "threaded"])
+def test_results_together_and_alone(sides):
+    """The same steps, times, centres of mass, fitness and travelled distance, bit for bit, whether
+    the engine finishes the simulations together (sizes below and above its threads' threshold) or
+    one at a time; and the same poses."""
+    import gpuvoxels_gb300 as g
+    docs = _docs(sides)
+
+    def fields(r):
+        return (r.steps, r.status, r.num_voxel, r.current_time, r.fitness_score, tuple(r.initial_center_of_mass),
+                tuple(r.current_center_of_mass), r.total_distance_of_all_voxels)
+
+    with g.Context(0, 512 << 20) as ctx:
+        ids = ctx.load_many(docs)
+        ctx.run(ids, g.BATCHED, 30)
+        together = [fields(ctx.result(i)) for i in ids]
+        pos, q, fl, off = ctx.get_states(ids)
+    alone = []
+    with g.Context(0, 512 << 20) as ctx:
+        for k, d in enumerate(docs):
+            i = ctx.load_vxa(d)
+            ctx.run(i, g.BATCHED, 30)
+            alone.append(fields(ctx.result(i)))
+            p, w, f = ctx.get_state(i)
+            assert np.array_equal(p, pos[off[k]:off[k + 1]]) and np.array_equal(w, q[off[k]:off[k + 1]])
+    assert together == alone
+    assert all(t[0] == 30 for t in together)
