@@ -302,10 +302,11 @@ public:
     int block_links_ = 256, block_voxels_ = 256, items_links_ = 1024, items_voxels_ = 1024, graph_steps_ = 64;
     int claim_links_ = 32, claim_voxels_ = 32;   // elements a warp claims from the step queues at a time
     // link binning: regrouped every bin_every_ steps (the first step after a batch change
-    // always); every second step measured 1.9% faster than every step on the 512-creature
-    // batch once it has settled (keys change slowly: 0.1% of links a step) and 1% faster on
-    // a fresh one, every fourth no faster than every second
-    int bin_every_ = 2, bin_phase_ = 0;
+    // always); a pass of 128 settled creatures takes 7.85, 7.52, 7.37 and 7.34 ms regrouped every
+    // step, second, fourth and eighth step, 512 fresh ones 25.1, 24.3, 24.2 and 24.9 ms, a slab
+    // 19.3, 19.1, 18.8 and 18.9 ms (keys change slowly: 0.1% of links a step once settled).  While
+    // more than 1 in 256 links change angle mode a step, every second step
+    int bin_every_ = 4, bin_phase_ = 0;
     bool bins_dirty_ = true;
     // Small batches (serving at low load) are bound by launch latency, not by the FP64 pipe:
     // their links and voxels are regrouped only when the batch changes and at the start of
@@ -403,7 +404,7 @@ public:
         device_ = device;
         CK(cudaSetDevice(device));
         CK(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device));
-        // GVX_LINK_BIN_EVERY: steps between regroupings of the links (tuning knob, default 1)
+        // GVX_LINK_BIN_EVERY: steps between regroupings of the links (tuning knob, default 4)
         if (const char* e = getenv("GVX_LINK_BIN_EVERY")) bin_every_ = std::max(1, atoi(e));
         CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         CK(cudaEventCreate(&ev0_));
@@ -1489,8 +1490,10 @@ public:
         const dev::Item* li = d_items_;
         const dev::Item* ci = d_items_ + n_link_items_;
         const dev::Item* vi = d_items_ + n_link_items_ + n_contact_items_;
-        const bool regroup = bins_dirty_ || (batch_links_ >= kRegroupEveryStepLinks && bin_phase_ % bin_every_ == 0);
-        if (regroup) {
+        const bool large = batch_links_ >= kRegroupEveryStepLinks;
+        const bool regroup = bins_dirty_ || (large && bin_phase_ % bin_every_ == 0);
+        const bool maybe = !regroup && large && bin_phase_ % 2 == 0;   // decided on the device
+        if (regroup || maybe) {
             // links and voxels grouped together (the voxel keys come from the last voxel
             // update, so nothing of this step changes them); windows of about 16k elements keep
             // a window's state in L2 while its key groups run
@@ -1498,9 +1501,10 @@ public:
                             d_link_total_, d_link_perm_};
             dev::BinList vb{vi, n_vox_items_, 1, std::max(1, 16384 / std::max(1, items_voxels_)), 0, d_vox_hist_, d_vox_base_,
                             d_vox_total_, d_vox_perm_};
-            ks_.bins(std::max(1, std::min(n_link_items_ + n_vox_items_, 4 * sm_count_)), st, d_sims_, d_ctl_, lb, vb);
+            ks_.bins(std::max(1, std::min(n_link_items_ + n_vox_items_, 4 * sm_count_)), st, d_sims_, d_ctl_, lb, vb, d_tickets_,
+                     maybe ? (int)std::min<size_t>(batch_links_, INT32_MAX) : 0);
             bins_dirty_ = false;
-            bin_phase_ = 0;
+            if (regroup) bin_phase_ = 0;
             launched += 3;
         }
         bin_phase_++;

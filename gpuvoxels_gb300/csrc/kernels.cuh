@@ -407,6 +407,14 @@ __device__ __forceinline__ int bin_key(const Sim& S, int kind, int begin, int j)
 #endif
 
 // ---------------------------------------------------------------- link binning
+// Whether a regrouping that is due only while links change angle mode is left out: at most one of the
+// batch's n_links in kBinRate did in the last step (tickets[6], which no kernel of the regrouping
+// writes: every block decides alike).  n_links 0: never.
+constexpr int kBinRate = 256;
+__device__ __forceinline__ bool bins_settled(const int* tickets, int n_links) {
+    return n_links > 0 && (long long)tickets[6] * kBinRate <= (long long)n_links;
+}
+
 // Every few steps the links of every running simulation are grouped by key within
 // windows of consecutive work items (three small passes: key counts per item, their
 // exclusive scan, a stable scatter of (simulation, link) pairs); keys change slowly,
@@ -418,8 +426,9 @@ __device__ __forceinline__ int bin_key(const Sim& S, int kind, int begin, int j)
 // barriers: warps of cheap small-angle links waited for warps of costly large-angle
 // ones.  Grouping across the whole batch at once made every key group a separate
 // pass over all link state and tripled k_links' DRAM traffic.)
-__global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, const Ctl* __restrict__ ctl, BinList la, BinList lb) {
+__global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, const Ctl* __restrict__ ctl, BinList la, BinList lb, const int* tickets, int n_links) {
     grid_wait();
+    if (bins_settled(tickets, n_links)) return;
     __shared__ int wc[kOrderKeys * 8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int g = blockIdx.x; g < la.n_items + lb.n_items; g += gridDim.x) {
@@ -453,8 +462,9 @@ __global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, 
 // by key, item by item, so base[item][key] = links of earlier windows + links of
 // smaller keys in the window + links of that key in earlier items of the window.
 // Each thread scans a contiguous run of that order; the runs are joined by a block scan.
-__global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb) {
+__global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const int* tickets, int n_links) {
     grid_wait();
+    if (bins_settled(tickets, n_links)) return;
     __shared__ int s_sum[1024];
     const BinList& L = blockIdx.x == 0 ? la : lb;   // one block per list
     const int* hist = L.hist;
@@ -496,8 +506,9 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb) {
     if (threadIdx.x == blockDim.x - 1) *total = s_sum[blockDim.x - 1];
 }
 
-__global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sims, const Ctl* __restrict__ ctl, BinList la, BinList lb) {
+__global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sims, const Ctl* __restrict__ ctl, BinList la, BinList lb, const int* tickets, int n_links) {
     grid_wait();
+    if (bins_settled(tickets, n_links)) return;
     __shared__ int wc[kOrderKeys * 8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const unsigned below = (1u << lane) - 1u;
@@ -1938,10 +1949,10 @@ inline void step_launch(void (*k)(P...), int grid, int block, cudaStream_t s, A.
     c.numAttrs = 1;
     cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
 }
-inline void l_bins(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, BinList la, BinList lb) {
-    step_launch(k_bin_hist, g, 256, s, sims, ctl, la, lb);
-    step_launch(k_bin_scan, 2, 1024, s, la, lb);
-    step_launch(k_bin_scatter, g, 256, s, sims, ctl, la, lb);
+inline void l_bins(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, BinList la, BinList lb, const int* tk, int n_links) {
+    step_launch(k_bin_hist, g, 256, s, sims, ctl, la, lb, tk, n_links);
+    step_launch(k_bin_scan, 2, 1024, s, la, lb, tk, n_links);
+    step_launch(k_bin_scatter, g, 256, s, sims, ctl, la, lb, tk, n_links);
 }
 inline void l_links(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, const int2* perm, const int* total, int cap, int n_slots,
                     int* tk, int claim) {

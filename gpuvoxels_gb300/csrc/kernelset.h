@@ -10,8 +10,10 @@ namespace gvx {
 struct KernelSet {
     const char* name;
     // groups the elements of the running simulations by key for two lists at once (links and
-    // voxels), in windows of work items
-    void (*bins)(int grid, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, dev::BinList links, dev::BinList voxels);
+    // voxels), in windows of work items; with n_links > 0 only while links of a batch of that
+    // many change angle mode (tickets[6] of them in the last step)
+    void (*bins)(int grid, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, dev::BinList links, dev::BinList voxels,
+                 const int* tickets, int n_links);
     // perm holds at most `cap` entries; entries name slots below n_slots; warps claim `claim`
     // entries at a time (a multiple of 32)
     void (*links)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
