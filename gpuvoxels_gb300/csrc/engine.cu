@@ -1516,7 +1516,7 @@ public:
         // the watch-list passes: a persistent grid of 256-thread blocks over the listed items' work units
         if (any_watch_) ks_.watch(4 * sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_, d_stale_items_, d_tickets_, d_batch_slots_,
                                   n_batch_);
-        if (any_collide_) ks_.contacts(grid_for(n_contact_items_, 128), 128, st, d_sims_, d_ctl_, ci, n_contact_items_, d_tickets_);
+        if (any_collide_) ks_.contacts(sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_);
         if (n_attach_) ks_.attach(st, d_sims_, d_ctl_, d_attach_slots_, n_attach_);
         if (prof) cudaEventRecord(evk_[2], st);
         if (prof) cudaEventRecord(evk_[3], st);

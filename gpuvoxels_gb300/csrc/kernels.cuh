@@ -679,8 +679,10 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
 }
 
 // Overlap test and repelling force for one voxel pair (CVX_Collision::updateContactForce,
-// Voxelyze3/src/old/VX_Collision.cpp:17-23, 42-56).  a < b; returns false when apart.
-__device__ __forceinline__ bool pair_force(const Sim& S, int a, int b, float* f3) {
+// Voxelyze3/src/old/VX_Collision.cpp:17-23, 42-56).  a < b; returns false when apart.  The plain form;
+// pair_force below takes the products and quotients to the integer pipes first (two of the about 60
+// FP64 instructions' worth were divisions; what stays are about a dozen sums).
+__device__ __forceinline__ bool pair_force_plain(const Sim& S, int a, int b, float* f3) {
     const VMat& ma = S.vm[__ldg(S.vmat + a)];
     const VMat& mb = S.vm[__ldg(S.vmat + b)];
     const float ox = d2f(S.px[b] - S.px[a]), oy = d2f(S.py[b] - S.py[a]), oz = d2f(S.pz[b] - S.pz[a]);
@@ -694,6 +696,34 @@ __device__ __forceinline__ bool pair_force(const Sim& S, int a, int b, float* f3
     const double vbx = S.mx[b] * mb.massInv, vby = S.my[b] * mb.massInv, vbz = S.mz[b] * mb.massInv;
     const double dux = f2d(ux), duy = f2d(uy), duz = f2d(uz);
     const float rv = d2f((vax * dux + vay * duy + vaz * duz) - (vbx * dux + vby * duy + vbz * duz));
+    const float k = 2.0f / (1.0f / ma.penStiff + 1.0f / mb.penStiff);
+    const float cd = 0.5f * (ma.cDampT + mb.cDampT);
+    const float f = k * relDist + cd * rv;
+    f3[0] = f * ux; f3[1] = f * uy; f3[2] = f * uz;
+    return true;
+}
+__device__ __noinline__ bool pair_force_rare(const Sim& S, int a, int b, float* f3) { return pair_force_plain(S, a, b, f3); }
+
+__device__ __forceinline__ bool pair_force(const Sim& S, int a, int b, float* f3) {
+    if (!kIntPipes) return pair_force_plain(S, a, b, f3);
+    IntPipes ip;
+    const VMat& ma = S.vm[__ldg(S.vmat + a)];
+    const VMat& mb = S.vm[__ldg(S.vmat + b)];
+    const float ox = d2f(S.px[b] - S.px[a]), oy = d2f(S.py[b] - S.py[a]), oz = d2f(S.pz[b] - S.pz[a]);
+    const double ba = ip.mul(ma.nom, ip.wide(1 + S.temp[a] * ma.cte)), bb = ip.mul(mb.nom, ip.wide(1 + S.temp[b] * mb.cte));
+    const float nomDist = ip.narrow(ip.mul(ip.div(mul2_band(ba) + ba, 3.0) + ip.div(mul2_band(bb) + bb, 3.0), ip.wide(S.env_radius)));
+    if (!ip.ok()) return pair_force_rare(S, a, b, f3);
+    const float len = sqrtf(ox * ox + oy * oy + oz * oz);
+    const float relDist = nomDist - len;
+    if (!(relDist > 0)) return false;
+    float ux = ox, uy = oy, uz = oz;
+    if (len > 0) { const float inv = 1.0f / len; ux = inv * ox; uy = inv * oy; uz = inv * oz; }
+    const double mia = ip.wide(ma.massInv), mib = ip.wide(mb.massInv);
+    const double dux = ip.wide(ux), duy = ip.wide(uy), duz = ip.wide(uz);
+    const double va = ip.mul0(ip.mul0(S.mx[a], mia), dux) + ip.mul0(ip.mul0(S.my[a], mia), duy) + ip.mul0(ip.mul0(S.mz[a], mia), duz);
+    const double vb = ip.mul0(ip.mul0(S.mx[b], mib), dux) + ip.mul0(ip.mul0(S.my[b], mib), duy) + ip.mul0(ip.mul0(S.mz[b], mib), duz);
+    const float rv = d2f(va - vb);
+    if (!ip.ok()) return pair_force_rare(S, a, b, f3);
     const float k = 2.0f / (1.0f / ma.penStiff + 1.0f / mb.penStiff);
     const float cd = 0.5f * (ma.cDampT + mb.cDampT);
     const float f = k * relDist + cd * rv;
@@ -1042,86 +1072,116 @@ __global__ void __launch_bounds__(256) k_watch_build(const Sim* __restrict__ sim
     });
 }
 
-// The contact pass of surface voxel v (surface index si) from its watch list: the list is in
-// increasing partner order, so the overlapping pairs (float envelope test, then the exact
-// test) are the reference's colWatch terms in order; their forces go straight to the voxel's
-// slots, and a voxel with more than its slots walks the list again into a spill run.
-__device__ void voxel_contacts_watch(const Sim& S, int v, int si, Ctl& c) {
+// The contact pass of surface voxel v (surface index si) from its watch list, by a group of G lanes of
+// one warp (all of which call it; g is the lane's place in the group, gmask the group's lanes): the
+// list is in increasing partner order, so the overlapping pairs (float envelope test, then the exact
+// test) are the reference's colWatch terms in order.  The lanes test G partners at a time, and a pair's
+// rank among the overlapping ones says where its force goes: the voxel's slots, or for a voxel with
+// more than its slots a spill run filled by a second walk.
+template <int G>
+__device__ void voxel_contacts_watch(const Sim& S, int v, int si, Ctl& c, int g, unsigned gmask) {
     const int cap = min(max(S.contact_inline, 1), kContactInline);
     float* out = S.cforce + (size_t)v * 3 * kContactInline;
     const float4 pv = S.cpos[v];
     int b = S.woff[2 * si], e = b + S.woff[2 * si + 1];
     if (b < 0 || e > S.wcap || b > e) {   // never: a run outside the lists is read as empty
-        atomicOr(&c.error, 4);
+        if (g == 0) atomicOr(&c.error, 4);
         b = e = 0;
     }
     const bool targets = S.flags & SF_TARGETS;
     const bool tv = targets && (S.vm[__ldg(S.vmat + v)].vx3 & VM_TARGET);
-    int n = 0, pairs = 0;
+    const unsigned below = gmask & ((1u << (threadIdx.x & 31)) - 1u);
+    int pairs = 0;
     bool hit = false;
-    for (int k = b; k < e; k++) {
-        const int q = S.wlist[k];
-        if ((unsigned)q >= (unsigned)S.nv) { atomicOr(&c.error, 4); continue; }   // never: not a voxel
-        if (!maybe_touching(pv, S.cpos[q], S.env_radius)) continue;
-        float f3[3];
-        if (!pair_force(S, v < q ? v : q, v < q ? q : v, f3)) continue;
-        if (n < cap) {
-            const float sgn = v < q ? 1.0f : -1.0f;   // contactForce(): +force on voxel1, -force on voxel2
-            out[3 * n] = sgn * f3[0]; out[3 * n + 1] = sgn * f3[1]; out[3 * n + 2] = sgn * f3[2];
+    // walks the list; put(rank, partner, force) for every overlapping pair; returns their number
+    auto walk = [&](auto put) {
+        int n = 0;
+        for (int k0 = b; k0 < e; k0 += G) {
+            const int k = k0 + g;
+            int q = k < e ? S.wlist[k] : -1;
+            if (k < e && (unsigned)q >= (unsigned)S.nv) { atomicOr(&c.error, 4); q = -1; }   // never: not a voxel
+            float f3[3];
+            const bool touch = q >= 0 && maybe_touching(pv, S.cpos[q], S.env_radius) && pair_force(S, v < q ? v : q, v < q ? q : v, f3);
+            const unsigned m = G == 1 ? (touch ? gmask : 0u) : __ballot_sync(gmask, touch) & gmask;
+            if (touch) put(n + __popc(m & below), q, f3);
+            n += __popc(m);
         }
-        n++;
+        return n;
+    };
+    const int n = walk([&](int r, int q, const float* f3) {
+        if (r < cap) {
+            const float sgn = v < q ? 1.0f : -1.0f;   // contactForce(): +force on voxel1, -force on voxel2
+            out[3 * r] = sgn * f3[0]; out[3 * r + 1] = sgn * f3[1]; out[3 * r + 2] = sgn * f3[2];
+        }
         if (targets && (bool)(S.vm[__ldg(S.vmat + q)].vx3 & VM_TARGET) != tv) { hit = true; if (q > v) pairs++; }
-    }
+    });
     if (n > cap) {
-        const int off = atomicAdd(S.spill_used, n);
+        int off = 0;
+        if (g == 0) off = atomicAdd(S.spill_used, n);
+        if (G > 1) off = __shfl_sync(gmask, off, 0, G);
         if (off < 0 || (unsigned)off > (unsigned)(S.spill_cap - n)) {
-            atomicOr(&c.error, 2);   // the pool's records for this step are used up
-            S.ccount[v] = 0;
+            if (g == 0) {
+                atomicOr(&c.error, 2);   // the pool's records for this step are used up
+                S.ccount[v] = 0;
+            }
             return;
         }
-        int j = 0;
-        for (int k = b; k < e && j < n; k++) {
-            const int q = S.wlist[k];
-            if ((unsigned)q >= (unsigned)S.nv) continue;
-            if (!maybe_touching(pv, S.cpos[q], S.env_radius)) continue;
-            float f3[3];
-            if (!pair_force(S, v < q ? v : q, v < q ? q : v, f3)) continue;
+        walk([&](int r, int q, const float* f3) {
+            if (r >= n) return;
             const float sgn = v < q ? 1.0f : -1.0f;
-            S.spill_p[off + j] = q;
-            float* o = S.spill_f + 3 * (size_t)(off + j);
+            S.spill_p[off + r] = q;
+            float* o = S.spill_f + 3 * (size_t)(off + r);
             o[0] = sgn * f3[0]; o[1] = sgn * f3[1]; o[2] = sgn * f3[2];
-            j++;
-        }
-        S.cspill[v] = off;
+        });
+        if (g == 0) S.cspill[v] = off;
     }
-    S.ccount[v] = n;
+    if (g == 0) S.ccount[v] = n;
     if (targets) {   // VX3 target contacts, as in voxel_contacts
         if (pairs) atomicAdd(&c.hit_count, pairs);
-        if (hit && !tv && (S.flags & SF_SIGNALS)) S.vfl[v] |= VF_TGTHIT;
+        if (G > 1) hit = __ballot_sync(gmask, hit) & gmask;
+        if (g == 0 && hit && !tv && (S.flags & SF_SIGNALS)) S.vfl[v] |= VF_TGTHIT;
     }
 }
 
-__global__ void __launch_bounds__(128) k_contacts(const Sim* __restrict__ sims, Ctl* ctl, const Item* __restrict__ items, int n_items, int* tickets) {
+// The contact items (at most 128 surface voxels each), a warp at a time in units of 32 / G voxels, one
+// voxel a group of G lanes; a simulation on the hash search takes one lane a voxel, an item in its
+// first four units.  No queue and no block barrier: units are short and much alike.
+//
+// Bound: latency.  Every partner is two dependent reads (list, position) and for the few that touch the
+// state of both, after five reads a voxel; a lane that walks its list alone takes as long as the longest
+// list.  Eight lanes a voxel where the warps are few: 37 -> 16 us for a settled 12^3 creature, 55 -> 20
+// for a 24^3 one, 57 -> 33 for a 40^3 one (31,000 surface voxels).  In a large batch they repeat the
+// reads a voxel for four voxels instead of 32 (249,000 surface voxels: 219 us against 117 settled), so
+// kContactWide surface voxels and fewer take them.  Seven blocks an SM: the integer-pipe pair test
+// at 96 registers and five blocks took 135 us there, at 64 and eight 119; the FP64 test 141.
+constexpr int kContactWide = 32768;
+template <int G>
+__global__ void __launch_bounds__(128, 7) k_contacts(const Sim* __restrict__ sims, Ctl* ctl, const Item* __restrict__ items, int n_items) {
     grid_wait();
-    __shared__ int s_item;
-    for (;;) {
-        const int it = claim(&tickets[1], &s_item);
-        if (it >= n_items) break;
-        const Item w = items[it];
+    constexpr int kUnits = 128 * G / 32;
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    const int g = lane % G;
+    const unsigned gmask = ((1u << G) - 1u) << (lane - g);
+    for (int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < n_items * kUnits; u += warps) {
+        const Item w = items[u / kUnits];
+        const int unit = u % kUnits;
         Ctl& c = ctl[w.sim];
         if (c.status != 1 || c.diverged) continue;
         const Sim& S = sims[w.sim];
         const int parity = c.hash_parity;
+        const bool watch = (S.flags & SF_WATCH) && c.watch_ok;
+        const int per_unit = watch ? 32 / G : 32;
+        const int ub = w.begin + unit * per_unit, ue = min(w.end, ub + per_unit);
+        if (ub >= ue) continue;
         // clear the other table for the insertions made by this step's voxel update
         int* other = S.hash_head + (size_t)(parity ^ 1) * S.hash_size;
         const int per = (S.hash_size + S.nsurf - 1) / (S.nsurf > 0 ? S.nsurf : 1);
-        const int cb = w.begin * per, ce = min(S.hash_size, (w.end == S.nsurf) ? S.hash_size : w.end * per);
-        for (int h = cb + threadIdx.x; h < ce; h += blockDim.x) other[h] = -1;
-        if ((S.flags & SF_WATCH) && c.watch_ok) {
-            for (int i = w.begin + threadIdx.x; i < w.end; i += blockDim.x) voxel_contacts_watch(S, S.surf[i], i, c);
-        } else {
-            for (int i = w.begin + threadIdx.x; i < w.end; i += blockDim.x) voxel_contacts(S, S.surf[i], parity, c);
-        }
+        const int cb = ub * per, ce = min(S.hash_size, (ue == S.nsurf) ? S.hash_size : ue * per);
+        for (int h = cb + lane; h < ce; h += 32) other[h] = -1;
+        const int i = ub + (watch ? lane / G : lane);
+        if (i >= ue) continue;
+        if (watch) voxel_contacts_watch<G>(S, S.surf[i], i, c, g, gmask);
+        else voxel_contacts(S, S.surf[i], parity, c);
     }
 }
 
@@ -1958,8 +2018,10 @@ inline void l_links(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, con
                     int* tk, int claim) {
     step_launch(k_links, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
 }
-inline void l_contacts(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n, int* tk) {
-    step_launch(k_contacts, g, b, s, sims, ctl, it, n, tk);
+inline void l_contacts(int sms, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n) {
+    // n items of at most 128 surface voxels; four warps a block
+    if (n <= kContactWide / 128) step_launch(k_contacts<8>, std::max(1, std::min(8 * n, 8 * sms)), 128, s, sims, ctl, it, n);
+    else step_launch(k_contacts<1>, std::max(1, std::min(n, 16 * sms)), 128, s, sims, ctl, it, n);
 }
 inline void l_watch(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n_items, const int* stale, const int* tk,
                     const int* slots, int n_sims) {

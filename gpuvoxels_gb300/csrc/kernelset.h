@@ -18,7 +18,7 @@ struct KernelSet {
     // entries at a time (a multiple of 32)
     void (*links)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
                   int n_slots, int* tickets, int claim);
-    void (*contacts)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n, int* tickets);
+    void (*contacts)(int sm_count, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n_items);
     void (*voxels)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
                    int n_slots, int* tickets, int claim);
     // the end of the step for n simulations (slot list): centre-of-mass sample, time, stop;

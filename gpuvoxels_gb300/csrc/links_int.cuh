@@ -25,6 +25,12 @@ namespace GVX_KNS {
 struct IntPipes {
     uint32_t rare = 0;
     __device__ __forceinline__ double mul(double x, double y) { return fp64i::mul_band(x, y, rare); }
+    // a product that may have an exact zero for a factor
+    __device__ __forceinline__ double mul0(double x, double y) {
+        const bool z = fp64i::eq0(x) | fp64i::eq0(y);
+        const double p = mul(z ? 1.0 : x, z ? 1.0 : y);
+        return z ? times_zero(x, y) : p;
+    }
     __device__ __forceinline__ double div(double x, double y) { return fp64i::div_band(x, y, rare); }
     __device__ __forceinline__ double root(double x) { return fp64i::sqrt_band(x, rare); }
     __device__ __forceinline__ double wide(float x) { return fp64i::f2d_band(x, rare); }

@@ -37,3 +37,25 @@ def test_results_together_and_alone(sides):
             assert np.array_equal(p, pos[off[k]:off[k + 1]]) and np.array_equal(w, q[off[k]:off[k + 1]])
     assert together == alone
     assert all(t[0] == 30 for t in together)
+
+
+@pytest.mark.parametrize("slots", [16, 1])
+def test_contacts_alone_and_in_a_large_batch(slots):
+    """A self-colliding creature's poses are the same bits whether its contact lists are walked by
+    eight lanes a voxel (alone) or by one (beside 60,000 other surface voxels); with one contact
+    slot a voxel every further contact goes through the spill pool."""
+    import gpuvoxels_gb300 as g
+    from gpuvoxels_gb300 import synth
+    mats = [dict(E=1e5, rho=1000.0, nu=0.35, cte=0.01, mus=1.0, muk=0.5), dict(E=1e6, rho=1000.0, nu=0.35, cte=0.0, mus=1.0, muk=0.5)]
+    small = [synth.random_creature(k, (12, 12, 12), 0.5, mats, collision=True, expansion=False).vxa for k in (3, 4)]
+    big = [synth.random_creature(k, (40, 40, 40), 0.5, mats, collision=True, expansion=False).vxa for k in (5, 6)]
+    poses = []
+    for docs in (small, small + big):
+        with g.Context(0, 2 << 30) as ctx:
+            ctx.set_contact_slots(slots)
+            ids = ctx.load_many(docs)
+            ctx.step(ids, 700)
+            pos, q, fl, off = ctx.get_states(ids)
+            n = off[2]
+            poses.append((pos[:n], q[:n], fl[:n]))
+    assert all(np.array_equal(a, b) for a, b in zip(*poses))
