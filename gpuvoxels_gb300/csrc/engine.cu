@@ -1473,6 +1473,9 @@ public:
     // them: the SM's one FP64 unit is what its warps share, so eight warps of one block cost a
     // small batch eight warps' time while other SMs idle (a 10^3 creature: k_links on 4 blocks
     // of 8 warps 40-44 us, on 31 blocks of one warp 34-37 us; the serving stream 41.3 -> 35.8 ms).
+    // The grid covers every SM even where there are fewer chunks: the warps that start first take
+    // them, and the pass of a 10^3 creature is 4 % shorter than with blocks for the chunks alone
+    // (2.81 -> 2.70 ms; a 12^3 colliding one 3.95 -> 3.85).
     struct Shape { int grid, block; };
     Shape grid_shape(size_t elems, int block, int claim, int which) {
         block = std::min(block, ks_.max_block);
@@ -1481,7 +1484,7 @@ public:
         const size_t want = (chunks + sms - 1) / sms;                                                // warps an SM
         if (want >= most * per_sm) return {(int)(sms * per_sm), block};
         const size_t blocks = (want + most - 1) / most, warps = (want + blocks - 1) / blocks;
-        return {(int)((chunks + warps - 1) / warps), (int)(32 * warps)};
+        return {(int)(sms * blocks), (int)(32 * warps)};
     }
 
     // One step of the batch; returns the number of kernels it launched.
