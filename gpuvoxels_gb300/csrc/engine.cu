@@ -1476,15 +1476,21 @@ public:
     // The grid covers every SM even where there are fewer chunks: the warps that start first take
     // them, and the pass of a 10^3 creature is 4 % shorter than with blocks for the chunks alone
     // (2.81 -> 2.70 ms; a 12^3 colliding one 3.95 -> 3.85).
-    struct Shape { int grid, block; };
+    struct Shape { int grid, block, depth; };   // depth: see KernelSet::links
     Shape grid_shape(size_t elems, int block, int claim, int which) {
         block = std::min(block, ks_.max_block);
         const size_t chunks = std::max<size_t>(1, (elems + claim - 1) / claim), sms = (size_t)sm_count_;
         const size_t per_sm = (size_t)ks_.resident_blocks(which, block), most = (size_t)block / 32;   // blocks an SM, warps a block
         const size_t want = (chunks + sms - 1) / sms;                                                // warps an SM
-        if (want >= most * per_sm) return {(int)(sms * per_sm), block};
+        // From kDeepRounds chunks a resident warp on, k_links takes its build for three blocks an SM (80
+        // registers): 512 creatures (19 chunks a warp) 24.4 -> 23.3 ms a pass, a slab (33) 18.1 -> 17.7;
+        // with five chunks a warp the longer tail costs more than it gives (128 creatures 7.29 -> 7.36 ms,
+        // eight colliding ones 8.25 -> 8.41).
+        constexpr size_t kDeepRounds = 10;
+        if (which == 0 && want >= kDeepRounds * most * per_sm) return {(int)(sms * ks_.resident_blocks(2, block)), block, 2};
+        if (want >= most * per_sm) return {(int)(sms * per_sm), block, 1};
         const size_t blocks = (want + most - 1) / most, warps = (want + blocks - 1) / blocks;
-        return {(int)(sms * blocks), (int)(32 * warps)};
+        return {(int)(sms * blocks), (int)(32 * warps), 0};
     }
 
     // One step of the batch; returns the number of kernels it launched.
@@ -1514,7 +1520,7 @@ public:
         if (prof) cudaEventRecord(evk_[0], st);
         // persistent grids; a batch that does not fill them is spread evenly over the SMs
         const Shape ls = grid_shape(batch_links_, block_links_, claim_links_, 0), vs = grid_shape(batch_voxels_, block_voxels_, claim_voxels_, 1);
-        ks_.links(ls.grid, ls.block, st, d_sims_, d_ctl_, d_link_perm_, d_link_total_, (int)cap_perm_, cap_slots_, d_tickets_, claim_links_);
+        ks_.links(ls.grid, ls.block, st, d_sims_, d_ctl_, d_link_perm_, d_link_total_, (int)cap_perm_, cap_slots_, d_tickets_, claim_links_, ls.depth);
         if (prof) cudaEventRecord(evk_[1], st);
         // the watch-list passes: a persistent grid of 256-thread blocks over the listed items' work units
         if (any_watch_) ks_.watch(4 * sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_, d_stale_items_, d_tickets_, d_batch_slots_,
@@ -1523,7 +1529,7 @@ public:
         if (n_attach_) ks_.attach(st, d_sims_, d_ctl_, d_attach_slots_, n_attach_);
         if (prof) cudaEventRecord(evk_[2], st);
         if (prof) cudaEventRecord(evk_[3], st);
-        ks_.voxels(vs.grid, vs.block, st, d_sims_, d_ctl_, d_vox_perm_, d_vox_total_, (int)cap_vperm_, cap_slots_, d_tickets_, claim_voxels_);
+        ks_.voxels(vs.grid, vs.block, st, d_sims_, d_ctl_, d_vox_perm_, d_vox_total_, (int)cap_vperm_, cap_slots_, d_tickets_, claim_voxels_, vs.depth);
         if (prof) cudaEventRecord(evk_[4], st);
         ks_.sim_end(st, d_sims_, d_ctl_, d_batch_slots_, n_batch_, d_tickets_, d_stale_items_);
         if (any_signals_) ks_.signals(grid_for(n_vox_items_, 256), 256, st, d_sims_, d_ctl_, vi, n_vox_items_, d_tickets_);

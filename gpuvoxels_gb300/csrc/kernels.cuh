@@ -10,6 +10,11 @@
 namespace gvx {
 namespace GVX_KNS {
 
+// 1.0 in a register of each lane, which the compiler cannot take for a constant or a uniform value
+// (see Add in links_int.cuh).
+__device__ double g_one[32] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
+__device__ __forceinline__ double opaque_one() { return *(volatile double*)&g_one[threadIdx.x & 31]; }
+
 // Whether links and voxels take the integer-pipe forms (links_int.cuh, voxels_int.cuh): the exact
 // build does; the FMA build's products contract with their sums on the FP64 pipe.
 #ifdef GVX_CONTRACT
@@ -567,11 +572,14 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sim
 constexpr int kLinkDefer = 48;          // a queue holds at most 31 + 16 links between rounds
 constexpr int kDeferPerWarp = 256;      // queues only with at least this many links per resident warp
 constexpr int kDeferRate = 256;         // queues while more than 1 link in kDeferRate changed mode
-__global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
+// F: sums by DFMA (see Add in links_int.cuh); B: resident blocks an SM the registers are sized for.
+template <bool F, int B>
+__global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
                                                                      const int* __restrict__ total, int cap, int n_slots, int* tickets,
                                                                      int claim) {
     grid_wait();
     __shared__ int2 s_defer[GVX_STEP_BLOCK / 32][2][kLinkDefer];   // per warp: large-angle (0), small-angle (1)
+    const double one = F ? opaque_one() : 1.0;
     // this step's queues of the kernels that follow, and the contact spill pool's records
     if (blockIdx.x == 0 && threadIdx.x == 0) { tickets[1] = 0; tickets[2] = 0; tickets[3] = 0; tickets[4] = 0; }
     const int n = min(*total, cap);
@@ -626,7 +634,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_LINKS_MIN_BLOCKS) k_links(
         // have stopped since the grouping was made
         bool act = e.x >= 0 && (unsigned)e.x < (unsigned)n_slots && ctl[e.x].status == 1 && (unsigned)e.y < (unsigned)sims[e.x].nl;
         LinkOrient o;
-        IntPipes ip;
+        IntPipes<F> ip(one);
         bool plain = false;      // this link takes the plain form (and is not deferred)
         if (kIntPipes) {
             if (act) {
@@ -706,7 +714,7 @@ __device__ __noinline__ bool pair_force_rare(const Sim& S, int a, int b, float* 
 
 __device__ __forceinline__ bool pair_force(const Sim& S, int a, int b, float* f3) {
     if (!kIntPipes) return pair_force_plain(S, a, b, f3);
-    IntPipes ip;
+    IntPipes<false> ip;
     const VMat& ma = S.vm[__ldg(S.vmat + a)];
     const VMat& mb = S.vm[__ldg(S.vmat + b)];
     const float ox = d2f(S.px[b] - S.px[a]), oy = d2f(S.py[b] - S.py[a]), oz = d2f(S.pz[b] - S.pz[a]);
@@ -1348,9 +1356,7 @@ __device__ __forceinline__ void voxel_update(const Sim& S, int v, float dt, cons
     q4 q = Q4(S.qw[v], S.qx[v], S.qy[v], S.qz[v]);
     d3 am = D3(S.ax[v], S.ay[v], S.az[v]);
     const float temp = S.temp[v];
-    bool fixed_all = false;
     if (e && (e->dof & 0x3F) == 0x3F) {
-        fixed_all = true;
         pos = D3(S.ijk[v] * m.nom + e->tr[0], S.ijk[nv + v] * m.nom + e->tr[1], S.ijk[2 * nv + v] * m.nom + e->tr[2]);
         q = Q4(e->rq[0], e->rq[1], e->rq[2], e->rq[3]);
         lm = am = D3(0, 0, 0);
@@ -1625,6 +1631,7 @@ __device__ __noinline__ void sim_control(const Sim& S, Ctl& c, bool div, double 
     if (stop) c.status = 2;
 }
 
+template <bool F>
 __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxels(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
                                                                        const int* __restrict__ total, int cap, int n_slots, int* tickets,
                                                                        int claim) {
@@ -1632,6 +1639,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
     // the voxels of the running simulations, grouped by key like the links (k_bin_*); warps
     // take chunks of `claim` voxels (a multiple of 32), so no warp waits at a block barrier
     // for a costlier one
+    const double one = F ? opaque_one() : 1.0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         tickets[0] = 0;
         tickets[6] = tickets[5];   // the last k_links launch's mode changes, for the next one
@@ -1669,7 +1677,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
             if (kIntPipes) {
                 const uint32_t fl = S.vfl[e.y];
                 bool plain = (S.flags & SF_VOXEL_EXTRAS) || (fl & VF_EXT) || ((fl & VF_PLAIN) && !plain_retry(c.steps));
-                if (!plain) plain = !voxel_update_int(S, e.y, fl, dt, st, S.flags, hnext, moved);
+                if (!plain) plain = !voxel_update_int<F>(S, e.y, fl, dt, st, S.flags, one, hnext, moved);
                 if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
             } else {
                 voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, moved);
@@ -2015,8 +2023,11 @@ inline void l_bins(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, BinList la,
     step_launch(k_bin_scatter, g, 256, s, sims, ctl, la, lb, tk, n_links);
 }
 inline void l_links(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, const int2* perm, const int* total, int cap, int n_slots,
-                    int* tk, int claim) {
-    step_launch(k_links, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
+                    int* tk, int claim, int depth) {
+    auto k = k_links<false, GVX_LINKS_MIN_BLOCKS>;
+    if (kIntPipes && depth == 1) k = k_links<kIntPipes, GVX_LINKS_MIN_BLOCKS>;
+    if (kIntPipes && depth == 2) k = k_links<kIntPipes, kIntPipes ? 3 : GVX_LINKS_MIN_BLOCKS>;
+    step_launch(k, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
 }
 inline void l_contacts(int sms, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n) {
     // n items of at most 128 surface voxels; four warps a block
@@ -2029,8 +2040,8 @@ inline void l_watch(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item
     step_launch(k_watch_build, g, 256, s, sims, ctl, it, n_items, stale, tk);
 }
 inline void l_voxels(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, const int2* perm, const int* total, int cap, int n_slots,
-                     int* tk, int claim) {
-    step_launch(k_voxels, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
+                     int* tk, int claim, int depth) {
+    step_launch(kIntPipes && depth ? k_voxels<kIntPipes> : k_voxels<false>, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
 }
 inline void l_sim_end(cudaStream_t s, const Sim* sims, Ctl* ctl, const int* slots, int n, int* tk, int* stale) {
     if (n > 0) step_launch(k_sim_end, n, 256, s, sims, ctl, slots, n, tk, stale);
@@ -2062,15 +2073,18 @@ inline void l_pack_results(cudaStream_t s, const Sim* sims, const int* slot, con
 inline void l_gather(cudaStream_t s, const Sim* sims, const int* slot, const int64_t* off, int n, int gx, double* pos3, double* q4, uint8_t* fl) {
     if (n > 0) k_gather<<<dim3((unsigned)gx, (unsigned)n), 256, 0, s>>>(sims, slot, off, n, pos3, q4, fl);
 }
-// Resident blocks per SM of the persistent grids at a block size (what the register use allows).
+// Resident blocks per SM of the persistent grids at a block size (what the register use allows):
+// k_links (0), k_voxels (1), k_links for deep batches (2).
 inline int l_resident_blocks(int which, int block) {
-    static int cached[2][33] = {};
+    static int cached[3][33] = {};
     block = block < 32 ? 32 : (block > 1024 ? 1024 : block & ~31);
-    int& n = cached[which ? 1 : 0][block >> 5];
+    which = which == 2 && kIntPipes ? 2 : (which == 1 ? 1 : 0);
+    int& n = cached[which][block >> 5];
     if (n == 0) {
         int r = 0;
-        if (which == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_links, block, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_voxels, block, 0);
+        if (which == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_links<kIntPipes, GVX_LINKS_MIN_BLOCKS>, block, 0);
+        else if (which == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_voxels<kIntPipes>, block, 0);
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_links<kIntPipes, kIntPipes ? 3 : GVX_LINKS_MIN_BLOCKS>, block, 0);
         n = r > 0 ? r : 1;
     }
     return n;

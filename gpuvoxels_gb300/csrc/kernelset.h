@@ -16,11 +16,12 @@ struct KernelSet {
                  const int* tickets, int n_links);
     // perm holds at most `cap` entries; entries name slots below n_slots; warps claim `claim`
     // entries at a time (a multiple of 32)
+    // depth: 0 not every resident warp has a chunk, 1 every one has, 2 (links) every one has many
     void (*links)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
-                  int n_slots, int* tickets, int claim);
+                  int n_slots, int* tickets, int claim, int depth);
     void (*contacts)(int sm_count, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n_items);
     void (*voxels)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
-                   int n_slots, int* tickets, int claim);
+                   int n_slots, int* tickets, int claim, int depth);
     // the end of the step for n simulations (slot list): centre-of-mass sample, time, stop;
     // simulations whose watch lists go stale append their contact items to stale_items
     // (count in tickets[7])
@@ -38,7 +39,7 @@ struct KernelSet {
     // n simulations (slot[k], output offset off[k]) into pos3 / q4 / flags (one launch).
     void (*gather)(cudaStream_t s, const dev::Sim* sims, const int* slot, const int64_t* off, int n, int gx, double* pos3, double* q4,
                    uint8_t* flags);
-    // resident blocks per SM of k_links (0) or k_voxels (1) at a block size
+    // resident blocks per SM of k_links (0), k_voxels (1) or k_links for deep batches (2) at a block size
     int (*resident_blocks)(int which, int block);
     int max_block;   // largest block k_links / k_voxels are compiled for
     // watch-list regeneration (one pass) of the simulations that need it: over the

@@ -17,13 +17,14 @@ namespace GVX_KNS {
 
 constexpr int SF_VOXEL_EXTRAS = SF_CILIA | SF_FFIELD | SF_SIGNALS | SF_ATTACH | SF_REMOVE | SF_FIXEDMAT;
 
-__device__ __forceinline__ q4 q_from_rotvec_int(IntPipes& a, const d3& v, bool* wide) {
+template <class Pipes>
+__device__ __forceinline__ q4 q_from_rotvec_int(Pipes& a, const d3& v, bool* wide) {
     const double tx = half_band(v.x), ty = half_band(v.y), tz = half_band(v.z);
     const double m2 = a.mul(tx, tx) + a.mul(ty, ty) + a.mul(tz, tz);
     double w, s;
     if (fp64i::lt_pos(a.mul(m2, m2), 5.328e-15)) {
-        w = 1.0 - half_band(m2);
-        s = 1.0 - a.div(m2, 6.0);
+        w = a.one - a.add(half_band(m2));
+        s = a.one - a.div(m2, 6.0);
     } else {
         *wide = true;
         const double m = a.root(m2);
@@ -35,9 +36,10 @@ __device__ __forceinline__ q4 q_from_rotvec_int(IntPipes& a, const d3& v, bool* 
 }
 
 // False: the voxel is left to the plain form, and nothing was stored.
-__device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t fl, float dt, const StepTimes& st, int flags, int* hash_next_table,
+template <bool kFma>
+__device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t fl, float dt, const StepTimes& st, int flags, double one, int* hash_next_table,
                                                  int* watch_moved) {
-    IntPipes a;
+    IntPipes<kFma> a(one);
     const int nv = S.nv;
     const VMat& m = S.vm[__ldg(S.vmat + v)];
     d3 pos = D3(S.px[v], S.py[v], S.pz[v]);
@@ -52,12 +54,12 @@ __device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t f
     d3 M = (fl & 1u) ? D3(sm[v], sm[nv + v], sm[2 * nv + v]) : D3(0, 0, 0);
 #pragma unroll
     for (int d = 1; d < 6; d++)
-        if (fl & (1u << d)) M = D3(M.x + sm[(d * 3) * nv + v], M.y + sm[(d * 3 + 1) * nv + v], M.z + sm[(d * 3 + 2) * nv + v]);
+        if (fl & (1u << d)) M = D3(a.add(M.x) + sm[(d * 3) * nv + v], a.add(M.y) + sm[(d * 3 + 1) * nv + v], a.add(M.z) + sm[(d * 3 + 2) * nv + v]);
     const double* sf = S.sf;
     d3 F = (fl & 1u) ? D3(sf[v], sf[nv + v], sf[2 * nv + v]) : D3(0, 0, 0);
 #pragma unroll
     for (int d = 1; d < 6; d++)
-        if (fl & (1u << d)) F = D3(F.x + sf[(d * 3) * nv + v], F.y + sf[(d * 3 + 1) * nv + v], F.z + sf[(d * 3 + 2) * nv + v]);
+        if (fl & (1u << d)) F = D3(a.add(F.x) + sf[(d * 3) * nv + v], a.add(F.y) + sf[(d * 3 + 1) * nv + v], a.add(F.z) + sf[(d * 3 + 2) * nv + v]);
     // one copy of the rotation for the two vectors, as in link_forces_int
     {
         d3 u = M;
@@ -83,9 +85,9 @@ __device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t f
     if (held) a.flag(!(fp64i::eq0(lm.x) && fp64i::eq0(lm.y)));   // so only before the first step
     if (m.gDampTD != 0) {
         const double gx = a.mul(m.gDampTD, vx), gy = a.mul(m.gDampTD, vy);
-        F = D3(F.x - (held ? 0.0 : gx), F.y - (held ? 0.0 : gy), F.z - a.mul(m.gDampTD, vz));
+        F = D3(a.add(F.x) - (held ? 0.0 : gx), a.add(F.y) - (held ? 0.0 : gy), F.z - a.mul(m.gDampTD, vz));
     }
-    F.z += m.gravForceD;
+    F.z = a.add(F.z) + m.gravForceD;
     if (flags & SF_COLLIDE) {
         const int nc = S.ccount[v];
         const float* cf = nc <= S.contact_inline ? S.cforce + (size_t)v * 3 * kContactInline : S.spill_f + 3 * (size_t)S.cspill[v];
@@ -96,19 +98,19 @@ __device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t f
     bool contact = false;
     if (flags & SF_FLOOR) {
         const double b = a.mul(m.nom, a.wide(1 + temp * m.cte));
-        const float pen = a.narrow(half_band(a.div(b + b + b, 3.0f)) - m.halfNom - pos.z);
+        const float pen = a.narrow(a.add(half_band(a.div(a.add(mul2_band(b)) + b, 3.0f))) - m.halfNom - pos.z);
         contact = pen >= 0;
         if (contact) {
             const float normal = m.penStiff * pen;
-            F.z += a.wide(normal) - (m.cDampTD != 0 ? a.mul(m.cDampTD, vz) : 0.0);
+            F.z = a.add(F.z) + (a.wide(normal) - (m.cDampTD != 0 ? (double)a.mul(m.cDampTD, vz) : 0.0));
             if (held) {
                 const float surf = d2f(a.mul(F.x, F.x) + a.mul(F.y, F.y)), fr = (m.mus * normal) * (m.mus * normal);
                 if (surf > fr) fl &= ~VF_STATIC;
             } else if (m.muk != 0) {
                 const double inv = a.div(1.0, a.root(a.mul(vx, vx) + a.mul(vy, vy)));
                 const double k = a.wide(m.muk * normal);
-                F.x -= a.mul(k, a.mul(inv, vx));
-                F.y -= a.mul(k, a.mul(inv, vy));
+                F.x = F.x - a.mul(k, a.mul(inv, vx));
+                F.y = F.y - a.mul(k, a.mul(inv, vy));
             }
         }
         fl = contact ? (fl | VF_FLOORC) : (fl & ~VF_FLOORC);
@@ -125,7 +127,7 @@ __device__ __forceinline__ bool voxel_update_int(const Sim& S, int v, uint32_t f
     }
     if (!a.ok()) return false;
 
-    pos = D3(pos.x + tr.x, pos.y + tr.y, pos.z + tr.z);
+    pos = D3(a.add(pos.x) + tr.x, a.add(pos.y) + tr.y, a.add(pos.z) + tr.z);
     S.px[v] = pos.x; S.py[v] = pos.y; S.pz[v] = pos.z;
     S.mx[v] = lm.x; S.my[v] = lm.y; S.mz[v] = lm.z;
     S.qw[v] = q.w; S.qx[v] = q.x; S.qy[v] = q.y; S.qz[v] = q.z;

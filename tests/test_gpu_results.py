@@ -59,3 +59,21 @@ def test_contacts_alone_and_in_a_large_batch(slots):
             n = off[2]
             poses.append((pos[:n], q[:n], fl[:n]))
     assert all(np.array_equal(a, b) for a, b in zip(*poses))
+
+
+@pytest.mark.parametrize("side", [34, 68], ids=["every_warp_busy", "many_chunks_a_warp"])
+def test_a_creature_beside_a_large_body(side):
+    """A creature's poses are the same bits alone (few warps an SM) and beside a solid body that gives
+    every resident warp a chunk of links, or many: the builds of the step kernels for those."""
+    import gpuvoxels_gb300 as g
+    from gpuvoxels_gb300 import synth
+    docs = [synth.config0_creature(6).vxa, synth.slab(side, side, side, seed=2).vxa]
+    poses = []
+    for d in (docs[:1], docs):
+        with g.Context(0, 2 << 30) as ctx:
+            ids = ctx.load_many(d)
+            ctx.step(ids, 40)
+            pos, q, fl, off = ctx.get_states(ids)
+            n = off[1]
+            poses.append((pos[:n], q[:n], fl[:n]))
+    assert all(np.array_equal(a, b) for a, b in zip(*poses))
