@@ -340,6 +340,32 @@ GVX_FP64I double sqrt_band(double x, uint32_t& rare) {
     return from_words((uint32_t)(q >> 32) + E, (uint32_t)q);
 }
 
+// n / d and sqrt(x) for any operands: the forms above, and the FP64 instructions for the rare rest.
+GVX_FP64I double div_any(double n, double d) {
+    uint32_t rare = 0;
+    double q = div_band(n, d, rare);
+    if (rare & kOutOfBand) {
+#ifdef __CUDA_ARCH__
+        asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(q) : "d"(n), "d"(d));
+#else
+        q = n / d;
+#endif
+    }
+    return q;
+}
+GVX_FP64I double sqrt_any(double x) {
+    uint32_t rare = 0;
+    double q = sqrt_band(x, rare);
+    if (rare & kOutOfBand) {
+#ifdef __CUDA_ARCH__
+        asm volatile("sqrt.rn.f64 %0, %1;" : "=d"(q) : "d"(x));
+#else
+        q = __builtin_sqrt(x);
+#endif
+    }
+    return q;
+}
+
 // x/2 and 2x for an x that mul_band, div_band or sqrt_band checks afterwards (in band: the
 // exponent steps; a zero, infinity or NaN stays out of band).
 GVX_FP64I double half_band(double x) { return from_words(hi32(x) - 0x100000u, lo32(x)); }

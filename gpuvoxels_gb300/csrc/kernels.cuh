@@ -181,7 +181,7 @@ __device__ __forceinline__ void link_finish(const Sim& S, int l, float dt, const
         a1v = D3(0, 0, 0);                  // ToRotationVector of the identity
     } else {
         // pos2.Length(), used by FromAngleToPosX's general branch and for the axial position
-        const double len = sqrt(pos2.x * pos2.x + pos2.y * pos2.y + pos2.z * pos2.z);
+        const double len = root(pos2.x * pos2.x + pos2.y * pos2.y + pos2.z * pos2.z);
         angle1 = q_from_angle_to_posx(angle1, pos2, len, &wide1);
         angle2 = qmul_x0(angle1, angle2);
         pos2 = D3(len - restLen, 0, 0);
@@ -210,7 +210,7 @@ __device__ __forceinline__ void link_finish(const Sim& S, int l, float dt, const
     }
 
     // updateStrain
-    const float axial = d2f(pos2.x / restLen);
+    const float axial = d2f(quo(pos2.x, restLen));
     float stress;
     strain = axial;
     if (m.linear) {
@@ -1417,9 +1417,9 @@ __device__ __forceinline__ void voxel_update(const Sim& S, int v, float dt, cons
                     const float fr = (m.mus * normal) * (m.mus * normal);
                     if (surf > fr) fl &= ~VF_STATIC;
                 } else {
-                    const double hl = sqrt(fp64i::plus_zero(vx * vx + vy * vy));   // + 0.0 * 0.0
+                    const double hl = root(fp64i::plus_zero(vx * vx + vy * vy));   // + 0.0 * 0.0
                     double nx = vx, ny = vy, nz = 0.0;
-                    if (fp64i::gt0(hl)) { const double inv = 1.0 / hl; nx = inv * vx; ny = inv * vy; nz = inv * 0.0; }
+                    if (fp64i::gt0(hl)) { const double inv = quo(1.0, hl); nx = inv * vx; ny = inv * vy; nz = inv * 0.0; }
                     const double k = f2d(m.muk * normal);
                     F = D3(F.x - k * nx, F.y - k * ny, F.z - k * nz);
                 }

@@ -40,6 +40,19 @@ using fp64i::zero_minus;
 using fp64i::minus_zero;
 using fp64i::times_zero;
 
+// Quotients and roots of the update.  The FMA build, whose products stay on the FP64 pipe, takes them
+// to the integer pipes too (a division costs that pipe seven instructions' time, a root eight; neither
+// contracts with anything); in the exact build these functions serve the plain forms alone.
+// Out of line: a branch here would end the caller's basic block, and which products contract would
+// change.
+#ifdef GVX_CONTRACT
+__device__ __noinline__ double quo(double n, double d) { return fp64i::div_any(n, d); }
+__device__ __noinline__ double root(double x) { return fp64i::sqrt_any(x); }
+#else
+__device__ __forceinline__ double quo(double n, double d) { return n / d; }
+__device__ __forceinline__ double root(double x) { return sqrt(x); }
+#endif
+
 // (float)(n/d) compared with a float threshold T, deciding with one multiply
 // unless n/d lies within 2^-20 (relative) of T, where the quotient is formed
 // exactly.  Outside that band the rounded float quotient cannot reach T, so the
@@ -126,12 +139,12 @@ __device__ __forceinline__ d3 q_to_rotvec(const q4& q, bool* wide = nullptr) {
     if (fp64i::ge(fabs(q.w), 1.0)) return D3(0, 0, 0);   // q.w >= 1 || q.w <= -1
     double sl = 1.0 - q.w * q.w;
     if (fp64i::lt(sl, 2.4e-3)) {
-        double s = sqrt((2 - mul2(q.w)) / sl);
+        double s = root(quo(2 - mul2(q.w), sl));
         return D3(kX0 ? times_zero(s, q.x) : mul2(q.x) * s, mul2(q.y) * s, mul2(q.z) * s);
     }
     if (wide) *wide = true;
     double a = acos(q.w);
-    double inv = 1.0 / sqrt(sl);
+    double inv = quo(1.0, root(sl));
     return D3(kX0 ? times_zero(inv, times_zero(a, q.x)) : (mul2(q.x) * a) * inv, (mul2(q.y) * a) * inv, (mul2(q.z) * a) * inv);
 }
 // Quat3D::FromRotationVector  Quat3D.h:128-143
@@ -142,14 +155,14 @@ __device__ __forceinline__ q4 q_from_rotvec(const d3& v, bool* wide = nullptr) {
     double w, s;
     if (fp64i::lt(m2 * m2, 5.328e-15)) {
         w = 1.0 - half(m2);
-        s = 1.0 - m2 / 6.0;
+        s = 1.0 - quo(m2, 6.0);
     } else {
         if (wide) *wide = true;
-        double m = sqrt(m2);
+        double m = root(m2);
         double sn, cs;
         sincos(m, &sn, &cs);
         w = cs;
-        s = sn / m;
+        s = quo(sn, m);
     }
     return Q4(w, tx * s, ty * s, tz * s);
 }
@@ -178,8 +191,8 @@ __device__ __forceinline__ q4 q_from_angle_to_posx(const q4& cur, const d3& r, d
     bool small_turn = by == 1 && bz == 1;
     double yox = 0, zox = 0;
     if (by != 0 && bz != 0) {
-        yox = r.y / r.x;
-        zox = r.z / r.x;
+        yox = quo(r.y, r.x);
+        zox = quo(r.z, r.x);
         small_turn = fp64i::lt(fabs(yox), 1.732e-2) && fp64i::lt(fabs(zox), 1.732e-2);   // |yox|, |zox| < 1.732e-2
     }
     if (small_turn) {
@@ -189,10 +202,10 @@ __device__ __forceinline__ q4 q_from_angle_to_posx(const q4& cur, const d3& r, d
     if (wide) *wide = true;
     const double l = len;
     double nx = r.x, ny = r.y, nz = r.z;
-    if (fp64i::gt0(l)) { double li = 1.0 / l; nx *= li; ny *= li; nz *= li; }
+    if (fp64i::gt0(l)) { double li = quo(1.0, l); nx *= li; ny *= li; nz *= li; }
     double theta = acos(nx);
     if (fp64i::gt(theta, 3.14159265358979 - 1e-7)) return Q4(0, 0, 1, 0);
-    double ami = 1.0 / sqrt(nz * nz + ny * ny);
+    double ami = quo(1.0, root(nz * nz + ny * ny));
     double a = half(theta);
     double sn, cs;
     sincos(a, &sn, &cs);
@@ -282,7 +295,7 @@ __device__ __forceinline__ float poisson_power(const VMat& m, float x) {
 __device__ __forceinline__ double base_size(const VMat& m, float temp) { return m.nom * f2d(1 + temp * m.cte); }
 __device__ __forceinline__ double base_size_avg(const VMat& m, float temp) {
     double b = base_size(m, temp);
-    return (b + b + b) / 3.0f;
+    return quo(b + b + b, 3.0f);
 }
 // CVX_Voxel::transverseArea  VX_Voxel.cpp:360-373  (psa, psb: the two transverse Poisson strains)
 __device__ __forceinline__ float voxel_tarea(const VMat& m, float psa, float psb) {

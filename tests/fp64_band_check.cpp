@@ -80,6 +80,10 @@ GVX_FP64I int one_case(uint64_t i, uint32_t* in_band) {
     // an operand that is zero, subnormal, infinite or NaN is always found
     const uint64_t odd[] = {0, kSign, 1, kInf, kInf | kSign, 0x7FF8000000000000ull};
     const double o = from_bits(odd[t % 6]);
+    // any operands
+    auto same = [](double p, double w) { return bits(p) == bits(w) || (p != p && w != w); };
+    if (!same(div_any(x, y), x / y) || !same(div_any(o, y), o / y) || !same(div_any(y, o), y / o)) bad++;
+    if (!same(sqrt_any(z), sqrt(z)) || !same(sqrt_any(x), sqrt(x)) || !same(sqrt_any(o), sqrt(o))) bad++;
     auto missed = [&]() { const bool m = (r & kOutOfBand) == 0; r = 0; return m; };
     (void)mul_band(o, y, r); if (missed()) bad++;
     (void)mul_band(y, half_band(o), r); if (missed()) bad++;
