@@ -73,22 +73,22 @@ def measured_peaks():
 # dram__bytes_write.sum / links).  profiles/fp64_counts_by_workload.md has the captures.
 FP64_COUNTS = {
     # batch of 512 creatures, step 288 (the settled window the line's value is timed over)
-    "batch": dict(per_link=655165600 / 1627115, per_voxel=195889184 / 844972,
-                  lanes_link=655165600 / 21707472, lanes_voxel=195889184 / 6829054,
-                  traffic_per_link=764864000 / 1627115, source="ncu, 512-creature batch, step 288"),
+    "batch": dict(per_link=308699104 / 1627115, per_voxel=86921632 / 844972,
+                  lanes_link=308699104 / 10684910, lanes_voxel=86921632 / 3139438,
+                  traffic_per_link=(431895040 + 671297024) / 1627115, source="ncu, 512-creature batch, step 288"),
     # 8 of the 64 collision creatures, mean of steps 201, 1001 and 1901 (the 2,000 timed steps)
-    "collide": dict(per_link=(149924800 + 139983552 + 137419616) / 3 / 373621,
-                    per_voxel=(64035808 + 59213696 + 58503680) / 3 / 249183,
-                    lanes_link=(149924800 + 139983552 + 137419616) / (5079772 + 4651183 + 4567875),
-                    lanes_voxel=(64035808 + 59213696 + 58503680) / (2291351 + 2149824 + 2144277),
-                    traffic_per_link=(180225280 + 181382912 + 181297408) / 3 / 373621,
+    "collide": dict(per_link=(70586144 + 64533024 + 63018592) / 3 / 373621,
+                    per_voxel=(30746112 + 27282656 + 26794624) / 3 / 249183,
+                    lanes_link=(70586144 + 64533024 + 63018592) / (2406790 + 2158689 + 2120036),
+                    lanes_voxel=(30746112 + 27282656 + 26794624) / (1132672 + 1044085 + 1047985),
+                    traffic_per_link=(191341312 + 188014560 + 188793472) / 3 / 373621,
                     source="ncu, 8 collision creatures 40^3, mean of steps 201, 1001, 1901"),
     # a 100x100x50 slab, mean of steps 201, 1001 and 1901
-    "slab": dict(per_link=(695043520 + 694503200 + 694274368) / 3 / 1480000,
-                 per_voxel=(117620192 + 117357888 + 117292448) / 3 / 500000,
-                 lanes_link=(695043520 + 694503200 + 694274368) / (22570878 + 22544145 + 22522796),
-                 lanes_voxel=(117620192 + 117357888 + 117292448) / (3896502 + 3879244 + 3875868),
-                 traffic_per_link=(420665344 + 421070336 + 421153792) / 3 / 1480000,
+    "slab": dict(per_link=(340309184 + 339917792 + 339795712) / 3 / 1480000,
+                 per_voxel=(54041344 + 53835072 + 53802912) / 3 / 500000,
+                 lanes_link=(340309184 + 339917792 + 339795712) / (11182512 + 11179330 + 11174281),
+                 lanes_voxel=(54041344 + 53835072 + 53802912) / (1713486 + 1701517 + 1700288),
+                 traffic_per_link=(663611392 + 667149568 + 668494080) / 3 / 1480000,
                  source="ncu, 100x100x50 slab, mean of steps 201, 1001, 1901"),
 }
 # steps a whole run of each workload takes (the batch: 0.5 s simulated at its creatures' time steps)
