@@ -303,7 +303,8 @@ __device__ __noinline__ bool link_plain(const Sim& S, int l, float dt) {
 // Steps at which links and voxels on the plain form try the integer-pipe form again.  Of a random
 // creature's links 45-63 % hold an exact zero before step 1, 0.01-1 % before step 4 and hardly one later:
 // from step 4 to 15 every step (waiting for the 16th left lanes of many warps on the plain form: a first
-// pass over 512 creatures 33.1 -> 31.2 ms, 64 creatures' first 20 steps with load and results 9.8 -> 9.5;
+// pass over 512 creatures 5-8 % faster in three runs, 33.1 -> 31.2 ms in one; 64 creatures' first 20 steps
+// with load and results 9.8 -> 9.5 and 9.6 ms, where two runs of one side differ by 1.5 %;
 // from step 3 or 2 on a solid slab gains 8 % each, random creatures lose as much), then every 16th, so
 // that a body with lasting zeros seldom pays for both forms.
 __device__ __forceinline__ bool plain_retry(int64_t step) { return (step >= 4 && step < 16) || (step & 15) == 0; }
