@@ -1719,13 +1719,17 @@ public:
         return 0;
     }
 
+    // The simulations of a call's ids, each once and resident.  An id given twice is one simulation:
+    // listed twice its voxels would be updated by two threads of a step, and its result be written by
+    // two of finish_many's.
     int prepare(const int64_t* ids, int n, std::vector<SimRec*>* rs, std::string* err) {
         std::vector<SimRec*> fresh, begun;
         std::unordered_set<SimRec*> seen;
         for (int i = 0; i < n; i++) {
             SimRec* r = find(ids[i]);
             if (!r) { *err = "unknown simulation id"; return -6; }
-            if (!r->resident && seen.insert(r).second) fresh.push_back(r);
+            if (!seen.insert(r).second) continue;
+            if (!r->resident) fresh.push_back(r);
             rs->push_back(r);
         }
         TraceClock tc;
