@@ -3,6 +3,7 @@
 #include "engine.h"
 #include "kernelset.h"
 #include "layout.cuh"
+#include "threads.h"
 
 #include <algorithm>
 #include <atomic>
@@ -1965,16 +1966,6 @@ public:
         return 0;
     }
     static constexpr size_t kThreadedVoxels = 8192;   // the work on fewer costs less than starting threads (about 80 us)
-
-    // Runs `work` on up to `most` threads, this one among them.
-    template <typename F>
-    static void run_threads(size_t most, const F& work) {
-        const size_t nt = std::max<size_t>(1, std::min<size_t>(most, std::max(1u, std::thread::hardware_concurrency())));
-        std::vector<std::thread> pool;
-        for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
-        work();
-        for (auto& t : pool) t.join();
-    }
 
     // ---------------------------------------------------------------- serving
     int submit(int64_t id, int64_t horizon, std::string* err) override {
