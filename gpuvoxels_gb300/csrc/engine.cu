@@ -306,8 +306,10 @@ public:
     // always); a pass of 128 settled creatures takes 7.85, 7.52, 7.37 and 7.34 ms regrouped every
     // step, second, fourth and eighth step, 512 fresh ones 25.1, 24.3, 24.2 and 24.9 ms, a slab
     // 19.3, 19.1, 18.8 and 18.9 ms (keys change slowly: 0.1% of links a step once settled).  While
-    // more than 1 in 256 links change angle mode a step, every second step
+    // more than 1 in 256 links change angle mode a step, every second step, unless the caller sets the
+    // period (GVX_LINK_BIN_EVERY)
     int bin_every_ = 4, bin_phase_ = 0;
+    bool bin_adapts_ = true;
     bool bins_dirty_ = true;
     // Small batches (serving at low load) are bound by launch latency, not by the FP64 pipe:
     // their links and voxels are regrouped only when the batch changes and at the start of
@@ -405,8 +407,9 @@ public:
         device_ = device;
         CK(cudaSetDevice(device));
         CK(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device));
-        // GVX_LINK_BIN_EVERY: steps between regroupings of the links (tuning knob, default 4)
-        if (const char* e = getenv("GVX_LINK_BIN_EVERY")) bin_every_ = std::max(1, atoi(e));
+        // GVX_LINK_BIN_EVERY: steps between regroupings of the links (tuning knob; default 4, and 2
+        // while many links change mode)
+        if (const char* e = getenv("GVX_LINK_BIN_EVERY")) { bin_every_ = std::max(1, atoi(e)); bin_adapts_ = false; }
         CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         CK(cudaEventCreate(&ev0_));
         CK(cudaEventCreate(&ev1_));
@@ -1502,7 +1505,7 @@ public:
         const dev::Item* vi = d_items_ + n_link_items_ + n_contact_items_;
         const bool large = batch_links_ >= kRegroupEveryStepLinks;
         const bool regroup = bins_dirty_ || (large && bin_phase_ % bin_every_ == 0);
-        const bool maybe = !regroup && large && bin_phase_ % 2 == 0;   // decided on the device
+        const bool maybe = !regroup && large && bin_adapts_ && bin_phase_ % 2 == 0;   // decided on the device
         if (regroup || maybe) {
             // links and voxels grouped together (the voxel keys come from the last voxel
             // update, so nothing of this step changes them); windows of about 16k elements keep
