@@ -17,7 +17,8 @@ __device__ __forceinline__ double opaque_one() { return *(volatile double*)&g_on
 
 // Whether links and voxels take the integer-pipe forms (links_int.cuh, voxels_int.cuh): the exact
 // build does; the FMA build's products contract with their sums on the FP64 pipe.
-#ifdef GVX_CONTRACT
+// GVX_PLAIN_FORMS (a test's build) takes the plain forms everywhere.
+#if defined(GVX_CONTRACT) || defined(GVX_PLAIN_FORMS)
 constexpr bool kIntPipes = false;
 #else
 constexpr bool kIntPipes = true;
