@@ -313,8 +313,13 @@ public:
     bool bins_dirty_ = true;
     // Small batches (serving at low load) are bound by launch latency, not by the FP64 pipe:
     // their links and voxels are regrouped only when the batch changes and at the start of
-    // every graph replay, not every step.
+    // every graph replay, or after as many steps, and before steps 4, 8 and 16 of the youngest simulation
+    // (elements leave the plain form when they are grouped).  The steps before the 16th are launched
+    // one by one: a graph of theirs would be replayed for later ones.
     static constexpr size_t kRegroupEveryStepLinks = 200000;
+    static constexpr int kRegroupSmall = 64, kYoungSteps = 16;
+    int young_left_ = 0;   // steps until no simulation of the running batch is in its first kYoungSteps
+    void set_young(int64_t youngest) { young_left_ = (int)std::max<int64_t>(0, kYoungSteps - youngest); }
     size_t batch_links_ = 0, batch_voxels_ = 0;
     int sm_count_ = 152;
     int profiling_ = 0;
@@ -1504,7 +1509,8 @@ public:
         const dev::Item* ci = d_items_ + n_link_items_;
         const dev::Item* vi = d_items_ + n_link_items_ + n_contact_items_;
         const bool large = batch_links_ >= kRegroupEveryStepLinks;
-        const bool regroup = bins_dirty_ || (large && bin_phase_ % bin_every_ == 0);
+        const int age = kYoungSteps - young_left_;   // of the youngest simulation
+        const bool regroup = bins_dirty_ || bin_phase_ % (large ? bin_every_ : kRegroupSmall) == 0 || (!large && (age == 4 || age == 8));
         const bool maybe = !regroup && large && bin_adapts_ && bin_phase_ % 2 == 0;   // decided on the device
         if (regroup || maybe) {
             // links and voxels grouped together (the voxel keys come from the last voxel
@@ -1521,6 +1527,7 @@ public:
             launched += 3;
         }
         bin_phase_++;
+        if (young_left_ > 0 && --young_left_ == 0 && !large) bins_dirty_ = true;
         if (prof) cudaEventRecord(evk_[0], st);
         // persistent grids; a batch that does not fill them is spread evenly over the SMs
         const Shape ls = grid_shape(batch_links_, block_links_, claim_links_, 0), vs = grid_shape(batch_voxels_, block_voxels_, claim_voxels_, 1);
@@ -1623,6 +1630,7 @@ public:
             for (size_t i = 0; i < rs.size(); i++) {
                 std::vector<int> one{rs[i]->slot};
                 if (int e = build_items(one, err)) return e;
+                set_young(steps0[i]);
                 if (exact_steps_ >= 0) {
                     for (int64_t k = 0; k < exact_steps_; k++) { timing_.launches += launch_step(stream_, false); }
                     continue;
@@ -1648,7 +1656,13 @@ public:
             }
             // a graph is captured only when a whole one will run: fewer steps than a graph holds
             // go out as single launches (a capture the GPU waits for would cost more)
-            const bool use_graph = exact_steps_ < 0 ? !profiling_ : (!profiling_ && exact_steps_ >= graph_steps_);
+            int64_t left = exact_steps_;
+            set_young(*std::min_element(steps0.begin(), steps0.end()));
+            while (young_left_ > 0 && left != 0) {
+                timing_.launches += launch_step(stream_, profiling_ != 0);
+                if (left > 0) left--;
+            }
+            const bool use_graph = exact_steps_ < 0 ? !profiling_ : (!profiling_ && left >= graph_steps_);
             if (!graph_ && use_graph) {
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -1665,7 +1679,6 @@ public:
             }
             if (exact_steps_ >= 0) {
                 // a known step count: whole graphs, then single steps for the remainder, no polling
-                int64_t left = exact_steps_;
                 while (left > 0) {
                     if (graph_ && !profiling_ && left >= graph_len_) {
                         CK(cudaGraphLaunch(graph_, stream_));
@@ -2053,6 +2066,7 @@ public:
                 tg.push_back(r->horizon > 0 ? r->horizon : 1000000);
             }
             if (int e3 = set_running(slots, tg, err)) return e3;
+            set_young(0);
             batch_dirty_ = true;
         }
         if (active_.empty()) return 0;
@@ -2065,7 +2079,9 @@ public:
             batch_dirty_ = false;
         }
         int k = std::max(1, chunk);
-        if (!graph_ || graph_len_ != k) {
+        const bool young = young_left_ > 0;
+        for (int s = 0; young && s < k; s++) timing_.launches += launch_step(stream_, false);
+        if (!young && (!graph_ || graph_len_ != k)) {
             if (graph_) { cudaGraphExecDestroy(graph_); graph_ = nullptr; }
             cudaGraph_t g;
             CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -2078,8 +2094,10 @@ public:
             cudaGraphDestroy(g);
             graph_len_ = k;
         }
-        CK(cudaGraphLaunch(graph_, stream_));
-        timing_.launches += graph_launches_;
+        if (!young) {
+            CK(cudaGraphLaunch(graph_, stream_));
+            timing_.launches += graph_launches_;
+        }
         std::vector<int32_t> st(active_.size());
         {
             int lo = INT32_MAX, hi = -1;

@@ -288,27 +288,52 @@ namespace gvx {
 namespace GVX_KNS {
 
 // The plain form of a whole link update, for a link that the integer-pipe form left (out of line:
-// rare once a body moves).  Sets LF_PLAIN, which keeps the link on this form until plain_retry, so
-// that a body with lasting zeros (an exact symmetry) does not pay for both forms every step.  True
-// when the link's strain diverged.
-__device__ __noinline__ bool link_plain(const Sim& S, int l, float dt) {
+// rare once a body moves).  Sets LF_PLAIN, which keeps the link on this form until a grouping finds it
+// link_ready.  True when the link's strain diverged; *switched: its angle mode changed.  B: resident
+// blocks an SM (one copy for each register budget of k_links).
+template <int B>
+__device__ __noinline__ bool link_plain(const Sim& S, int l, float dt, bool* switched) {
     LinkOrient o;
     bool div = false;
+    *switched = false;
     if (link_orient(S, l, &o)) {
+        *switched = o.switched;
         link_finish(S, l, dt, o, &div);
         S.lfl[l] |= LF_PLAIN;
     }
     return div;
 }
 
-// Steps at which links and voxels on the plain form try the integer-pipe form again.  Of a random
-// creature's links 45-63 % hold an exact zero before step 1, 0.01-1 % before step 4 and hardly one later:
-// from step 4 to 15 every step (waiting for the 16th left lanes of many warps on the plain form: a first
-// pass over 512 creatures 5-8 % faster in three runs, 33.1 -> 31.2 ms in one; 64 creatures' first 20 steps
-// with load and results 9.8 -> 9.5 and 9.6 ms, where two runs of one side differ by 1.5 %;
-// from step 3 or 2 on a solid slab gains 8 % each, random creatures lose as much), then every 16th, so
-// that a body with lasting zeros seldom pays for both forms.
-__device__ __forceinline__ bool plain_retry(int64_t step) { return (step >= 4 && step < 16) || (step & 15) == 0; }
+// Links and voxels on the plain form go back to the integer-pipe form when the numbers whose exact
+// zeros sent them there are well inside the band (the products of two such are in band too).  A warp with
+// lanes on either form runs both.  So that is looked at when elements are grouped, where those that
+// change forms change warps as well, and between groupings in warps that run both forms anyway.  Groupings
+// look at a simulation's elements up to its 16th step and then in one of 16 steps at most: an element
+// that fails for a reason which the look does not see pays for both forms no oftener.
+// Against the plain kernels alone, steps 4 to 15 of a body whose zeros last or recede slowly (equal
+// phases, 110,592 voxels) went from 1.33 of their time, with a trial every step, to 1.07 (the rest: barriers
+// and calls around the plain form), 64 cantilevers' steps from 1.04-1.07 to 0.72.
+__device__ __forceinline__ bool plain_retry(const Ctl& c) { return c.steps <= 16 || c.steps - c.plain_at >= 16; }
+__device__ __forceinline__ bool sizable(double x) { return (fp64i::hi32(x) & 0x7FF00000u) - ((1023u - 110u) << 20) < (220u << 20); }   // 2^-110..2^110
+
+// The rotations of both voxels, and of the link's last pose what its mode does not make zero.
+__device__ __forceinline__ bool link_ready(const Sim& S, int l, uint8_t fl) {
+    const int ng = __ldg(S.lneg + l), pv = __ldg(S.lpos + l), nl = S.nl;
+    const double* st = S.lst + l;
+    const int at = fl & LF_SMALL ? 1 : 4;   // pos2's or angle1v's y and z
+    return sizable(st[6 * nl]) & sizable(st[7 * nl]) & sizable(st[8 * nl]) & sizable(st[at * nl]) & sizable(st[(at + 1) * nl]) &&
+           sizable(S.qx[ng]) & sizable(S.qy[ng]) & sizable(S.qz[ng]) & sizable(S.qx[pv]) & sizable(S.qy[pv]) & sizable(S.qz[pv]);
+}
+
+// The voxel's rotation and momenta (static friction holds the horizontal momentum at zero, which the
+// integer-pipe form expects).
+__device__ __forceinline__ bool voxel_ready(const Sim& S, int v, uint32_t fl) {
+    return sizable(S.ax[v]) & sizable(S.ay[v]) & sizable(S.az[v]) & sizable(S.mz[v]) &&
+           sizable(S.qx[v]) & sizable(S.qy[v]) & sizable(S.qz[v]) & ((fl & VF_STATIC) || (sizable(S.mx[v]) & sizable(S.my[v])));
+}
+// Voxels that never take the integer-pipe form.
+constexpr int SF_VOXEL_EXTRAS = SF_CILIA | SF_FFIELD | SF_SIGNALS | SF_ATTACH | SF_REMOVE | SF_FIXEDMAT;
+__device__ __forceinline__ bool always_plain(int flags, uint32_t fl) { return (flags & SF_VOXEL_EXTRAS) || (fl & VF_EXT); }
 
 // Work-item elements in an order that keeps warps on one code path.  GB300's FP64
 // pipe spends the same cycles on a warp instruction whatever its active lanes, so a
@@ -318,7 +343,7 @@ __device__ __forceinline__ bool plain_retry(int64_t step) { return (step >= 4 &&
 // deterministic.  The order never changes results: every link writes only its own
 // state and its two direction slots, and voxel work is per voxel.
 constexpr int kOrderMax = 1024;   // elements per item that are reordered (larger items run in index order)
-constexpr int kOrderKeys = kOrderKeysBins;
+constexpr int kOrderKeys = kIntPipes ? kOrderKeysBins : kOrderKeysBins / 2;   // one half for each form (see LinkKey)
 
 // perm[0..n) = element indices grouped by key(j) in increasing key order; wc holds
 // kOrderKeys x 8 warp counts.  Every thread of the block must call it.
@@ -368,23 +393,27 @@ __device__ __forceinline__ void order_by_key(int n, KeyFn key, int* perm, int* w
     }
 }
 
+// The keys' upper half are elements of the integer-pipe forms, the lower half those on the plain form
+// (the FMA build has one form and one half).  A warp with one lane on the plain form runs both: 64
+// cantilevers whose fixed voxels, and the links at them, keep to it took 273 us a step with forms
+// mixed and 184 apart.
+constexpr int kFormKeys = kOrderKeysBins / 2;
+
 // Link key: small-angle mode, then within each mode which rotation branches were taken
 // (small links: angle2's rotation-vector branch; large links: that, angle1's, and
-// FromAngleToPosX's).  10 groups, the costliest first (large links taking every
-// acos/sincos branch are key 0, plain small links key 9).
+// FromAngleToPosX's, which angle1's acos branch implies).  Eight groups a form, the costliest first
+// (large links taking every acos/sincos branch are key 0, plain small links key 7).
 struct LinkKey {
     const uint8_t* lfl;
     int begin;
     __device__ int operator()(int j) const {
         const uint8_t f = lfl[begin + j];
-        if (f & LF_SMALL) return (f & LF_WIDE2) ? 8 : 9;
-        return 7 - (((f & LF_WIDE1) ? 4 : 0) | ((f & LF_ACOS1) ? 2 : 0) | ((f & LF_WIDE2) ? 1 : 0));
+        const int wide2 = f & LF_WIDE2 ? 1 : 0;
+        const int k = f & LF_SMALL ? 7 - wide2 : 5 - 2 * (f & LF_ACOS1 ? 2 : (f & LF_WIDE1 ? 1 : 0)) - wide2;
+        return (!kIntPipes || (f & LF_PLAIN) ? 0 : kFormKeys) + k;
     }
 };
 
-// Voxel key: touched the floor last step (contact and friction branches) and, if so,
-// held by static friction (the kinetic branch forms the sliding direction), then
-// surface voxels (Poisson strain by pow) apart from interior ones.
 // Voxel key: floor contact with kinetic (0, 1) or static (2, 3) friction, else surface
 // (4, 6) or interior (5, 7) voxel; the lower key of each pair when the last orientation
 // update took the sin/cos branch.  (Voxels touching the floor are not told apart by
@@ -395,14 +424,25 @@ struct VoxelKey {
     __device__ int operator()(int j) const {
         const uint32_t f = vfl[begin + j];
         const int narrow = (f & VF_WROT) ? 0 : 1;
-        if (f & VF_FLOORC) return ((f & VF_STATIC) ? 2 : 0) + narrow;
-        return 4 + 2 * narrow + ((f & VF_INTERIOR) ? 1 : 0);
+        const int k = f & VF_FLOORC ? ((f & VF_STATIC) ? 2 : 0) + narrow : 4 + 2 * narrow + ((f & VF_INTERIOR) ? 1 : 0);
+        return (!kIntPipes || (f & VF_PLAIN) ? 0 : kFormKeys) + k;
     }
 };
 
 // Grouping key of element j of a work item starting at `begin`: links (kind 0) or voxels (kind 1).
 __device__ __forceinline__ int bin_key(const Sim& S, int kind, int begin, int j) {
     return kind == 0 ? LinkKey{S.lfl, begin}(j) : VoxelKey{S.vfl, begin}(j);
+}
+
+// Takes an element that is ready for it off the plain form.
+__device__ __forceinline__ void leave_plain(const Sim& S, int kind, int at) {
+    if (kind == 0) {
+        const uint8_t f = S.lfl[at];
+        if ((f & LF_PLAIN) && link_ready(S, at, f)) S.lfl[at] = f & ~LF_PLAIN;
+    } else {
+        const uint32_t f = S.vfl[at];
+        if ((f & VF_PLAIN) && !always_plain(S.flags, f) && voxel_ready(S, at, f)) S.vfl[at] = f & ~VF_PLAIN;
+    }
 }
 
 // Resident blocks per SM the register allocation of k_links / k_voxels is sized for
@@ -451,9 +491,11 @@ __global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, 
         const bool run = ctl[w.sim].status == 1;
         const Sim& S = sims[w.sim];
         const int n = w.end - w.begin;
+        const bool retry = kIntPipes && run && plain_retry(ctl[w.sim]);
         int cnt = 0;   // thread k < kOrderKeys: elements of key k
         for (int j0 = 0; j0 < n; j0 += blockDim.x) {
             const int j = j0 + threadIdx.x;
+            if (retry && j < n) leave_plain(S, kind, w.begin + j);
             const int kj = (run && j < n) ? bin_key(S, kind, w.begin, j) : -1;
 #pragma unroll
             for (int k = 0; k < kOrderKeys; k++) {
@@ -492,6 +534,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const
         return w * win + (r - *k * win);
     };
     int sum = 0;
+#pragma unroll 8
     for (int e = e0; e < e1; e++) {
         int k;
         const int it = item_of(e, &k);
@@ -506,6 +549,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const
         __syncthreads();
     }
     int run = threadIdx.x ? s_sum[threadIdx.x - 1] : 0;
+#pragma unroll 8
     for (int e = e0; e < e1; e++) {
         int k;
         const int it = item_of(e, &k);
@@ -517,10 +561,10 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const
     if (threadIdx.x == blockDim.x - 1) *total = s_sum[blockDim.x - 1];
 }
 
-__global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sims, const Ctl* __restrict__ ctl, BinList la, BinList lb, const int* tickets, int n_links) {
+__global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sims, Ctl* ctl, BinList la, BinList lb, const int* tickets, int n_links) {
     grid_wait();
     if (bins_settled(tickets, n_links)) return;
-    __shared__ int wc[kOrderKeys * 8];
+    __shared__ int wc[kOrderKeys * 8], start[kOrderKeys];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     for (int g = blockIdx.x; g < la.n_items + lb.n_items; g += gridDim.x) {
@@ -531,9 +575,11 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sim
         int2* perm = first ? la.perm : lb.perm;
         const Item w = (first ? la.items : lb.items)[it];
         if (ctl[w.sim].status != 1) continue;   // the same for the whole block
+        if (kIntPipes && kind == 1 && w.begin == 0 && threadIdx.x == 0 && plain_retry(ctl[w.sim])) ctl[w.sim].plain_at = ctl[w.sim].steps;
         const Sim& S = sims[w.sim];
-        int start[kOrderKeys];
-        for (int k = 0; k < kOrderKeys; k++) start[k] = base[(size_t)it * kOrderKeys + k];
+        // where each key's next element goes; in shared memory (as an array a thread, indexed by its key,
+        // it lay in local memory: 128 creatures 22.2 us, now 11.6)
+        if (threadIdx.x < kOrderKeys) start[threadIdx.x] = base[(size_t)it * kOrderKeys + threadIdx.x];
         const int n = w.end - w.begin;
         for (int j0 = 0; j0 < n; j0 += blockDim.x) {
             const int j = j0 + threadIdx.x;
@@ -551,8 +597,9 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sim
                 for (int q = 0; q < wid; q++) p += wc[kj * 8 + q];
                 perm[p] = make_int2(w.sim, w.begin + j);
             }
-            for (int k = 0; k < kOrderKeys; k++)
-                for (int q = 0; q < nw; q++) start[k] += wc[k * 8 + q];
+            __syncthreads();
+            if (threadIdx.x < kOrderKeys)
+                for (int q = 0; q < nw; q++) start[threadIdx.x] += wc[threadIdx.x * 8 + q];
             __syncthreads();
         }
     }
@@ -647,8 +694,14 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
                 const Sim& S = sims[e.x];
                 const uint8_t fl = S.lfl[e.y];
                 act = !(fl & LF_GONE) && !((S.flags & SF_FIXEDMAT) && fixed_link(S, e.y));
-                plain = (fl & LF_PLAIN) && !plain_retry(ctl[e.x].steps);
-                if (act && !plain) {
+                plain = (fl & LF_PLAIN) || ctl[e.x].steps == 0;   // at rest before step 0, every link holds zeros
+            }
+            const bool both = __ballot_sync(0xffffffffu, act && !plain) != 0;
+            if (act) {
+                const Sim& S = sims[e.x];
+                const uint8_t fl = S.lfl[e.y];
+                if (plain && both && (fl & LF_PLAIN)) plain = !link_ready(S, e.y, fl);
+                if (!plain) {
                     link_orient_int(ip, S, e.y, fl, &o);
                     plain = !ip.ok();
                 }
@@ -680,8 +733,10 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
             if (act && !plain) plain = !link_pose_int(ip, sims[e.x], e.y, o, &p);
             __syncthreads();
             if (act && !plain) plain = !link_forces_int(ip, sims[e.x], e.y, ctl[e.x].dt, p, &div);
-            if (act && plain) div = link_plain(sims[e.x], e.y, ctl[e.x].dt);
+            bool turned = false;
+            if (act && plain) div = link_plain<B>(sims[e.x], e.y, ctl[e.x].dt, &turned);
             if (div) ctl[e.x].diverged = 1;
+            switched += __popc(__ballot_sync(0xffffffffu, turned));
         } else if (act) {
             Ctl& c = ctl[e.x];
             bool div = false;
@@ -1670,10 +1725,25 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
         int2 e = make_int2(-1, -1);
         if (k + lane < k1) e = __ldg(perm + k + lane);
         k += 32;
-        if ((unsigned)e.x >= (unsigned)n_slots) continue;   // none, or never: the grouping lists running slots
-        const Ctl& c = ctl[e.x];
-        const float dt = c.dt;
-        if (c.status == 1 && !c.diverged && dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv) {
+        // e.x >= n_slots: none, or never (the grouping lists running slots)
+        bool act = (unsigned)e.x < (unsigned)n_slots;
+        if (act) {
+            const Ctl& c = ctl[e.x];
+            act = c.status == 1 && !c.diverged && c.dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv;
+        }
+        uint32_t fl = 0;
+        bool plain = false;
+        if (kIntPipes) {
+            if (act) {
+                fl = sims[e.x].vfl[e.y];
+                plain = (fl & VF_PLAIN) || always_plain(sims[e.x].flags, fl) || ctl[e.x].steps == 0;
+            }
+            const bool both = __ballot_sync(0xffffffffu, act && !plain) != 0;
+            if (plain && both && (fl & VF_PLAIN) && !always_plain(sims[e.x].flags, fl)) plain = !voxel_ready(sims[e.x], e.y, fl);
+        }
+        if (act) {
+            const Ctl& c = ctl[e.x];
+            const float dt = c.dt;
             const Sim& S = sims[e.x];
             StepTimes st;
             st.t_now = c.t; st.t_next = c.t + dt; st.t_cycles = c.t_cycles; st.angle = c.recent_angle;
@@ -1681,8 +1751,6 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
             int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
             int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
             if (kIntPipes) {
-                const uint32_t fl = S.vfl[e.y];
-                bool plain = (S.flags & SF_VOXEL_EXTRAS) || (fl & VF_EXT) || ((fl & VF_PLAIN) && !plain_retry(c.steps));
                 if (!plain) plain = !voxel_update_int<F>(S, e.y, fl, dt, st, S.flags, one, hnext, moved);
                 if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
             } else {

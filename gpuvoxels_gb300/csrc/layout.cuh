@@ -16,7 +16,7 @@ namespace dev {
 // budget, limits the contacts of a whole step).
 constexpr int kContactInline = 16;
 constexpr int kReachWords = 8;        // 231 offsets of the L1 ball of radius 5 -> 8 x 32 bits
-constexpr int kOrderKeysBins = 10;    // link ordering keys (the step kernels' kOrderKeys)
+constexpr int kOrderKeysBins = 16;    // link and voxel ordering keys (the step kernels' kOrderKeys)
 
 // voxel flag bits
 constexpr uint32_t VF_LINKS = 0x3Fu;      // bits 0..5: link present in direction d
@@ -32,13 +32,13 @@ constexpr uint8_t LF_WIDE2 = 8;           // last step: angle2's rotation vector
 constexpr uint8_t LF_ACOS1 = 16;          // last step: angle1's rotation vector took the acos branch
 constexpr uint8_t LF_GONE = 32;           // VX3: detached (failed) or removed with a voxel: no longer updated
 constexpr uint8_t LF_REMOVED = 64;        // VX3: removed with a voxel (left out of the history's link records)
-constexpr uint8_t LF_PLAIN = 128;         // last step: taken by the plain form of the update (not shown to callers)
+constexpr uint8_t LF_PLAIN = 128;         // on the plain form of the update (not shown to callers)
 constexpr uint32_t VF_FLOORC = 1u << 10;  // last step: the voxel touched the floor
 constexpr uint32_t VF_REMOVED = 1u << 11; // VX3: removed from the simulation (frozen, no links, no contacts)
 constexpr uint32_t VF_TGTHIT = 1u << 12;  // VX3: this step's contacts include a target voxel (non-target voxel)
 constexpr uint32_t VF_ATTACH = 1u << 13;  // VX3: enableAttach (every attach condition holds at the voxel)
 constexpr uint32_t VF_WROT = 1u << 14;    // last step: the orientation update took the sin/cos branch (grouping key only)
-constexpr uint32_t VF_PLAIN = 1u << 15;   // last step: taken by the plain form of the update (not shown to callers)
+constexpr uint32_t VF_PLAIN = 1u << 15;   // on the plain form of the update (not shown to callers)
 
 // sim flag bits
 constexpr int SF_FLOOR = 1, SF_COLLIDE = 2, SF_VARY = 4, SF_EXPAND = 8;
@@ -222,6 +222,7 @@ struct Ctl {
     int32_t c_item_count;
     int32_t watch_used;         // SF_WATCH: list entries taken by this regeneration's runs
     int32_t pad_watch;
+    int64_t plain_at;           // the step whose grouping last looked at the elements on the plain form
     double init_com[3];         // initial centre of mass (host value, reset by the secondary experiment)
     MathTree stop;
 };

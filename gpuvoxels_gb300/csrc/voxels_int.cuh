@@ -6,7 +6,7 @@
 //
 // It takes voxels without an external in simulations without the VX3 extras that act on voxels;
 // others go to the plain form at once.  A voxel with an operand out of band is left to the plain
-// form before anything is stored; VF_PLAIN keeps it there until plain_retry.  The horizontal
+// form before anything is stored; VF_PLAIN keeps it there until it is voxel_ready.  The horizontal
 // momentum of a voxel held by static friction is exactly zero: its products stand in with 1 and
 // are not used.
 #pragma once
@@ -14,8 +14,6 @@
 
 namespace gvx {
 namespace GVX_KNS {
-
-constexpr int SF_VOXEL_EXTRAS = SF_CILIA | SF_FFIELD | SF_SIGNALS | SF_ATTACH | SF_REMOVE | SF_FIXEDMAT;
 
 template <class Pipes>
 __device__ __forceinline__ q4 q_from_rotvec_int(Pipes& a, const d3& v, bool* wide) {
