@@ -454,13 +454,13 @@ public:
         cap_attach_ = 1024;
         CK(cudaMalloc(&d_link_hist_, sizeof(int) * cap_bins_));
         CK(cudaMalloc(&d_link_base_, sizeof(int) * cap_bins_));
-        CK(cudaMalloc(&d_link_total_, sizeof(int)));
-        CK(cudaMemset(d_link_total_, 0, sizeof(int)));
+        CK(cudaMalloc(&d_link_total_, 2 * sizeof(int)));
+        CK(cudaMemset(d_link_total_, 0, 2 * sizeof(int)));
         CK(cudaMalloc(&d_link_perm_, sizeof(int2) * cap_perm_));
         CK(cudaMalloc(&d_vox_hist_, sizeof(int) * cap_vbins_));
         CK(cudaMalloc(&d_vox_base_, sizeof(int) * cap_vbins_));
-        CK(cudaMalloc(&d_vox_total_, sizeof(int)));
-        CK(cudaMemset(d_vox_total_, 0, sizeof(int)));
+        CK(cudaMalloc(&d_vox_total_, 2 * sizeof(int)));
+        CK(cudaMemset(d_vox_total_, 0, 2 * sizeof(int)));
         CK(cudaMalloc(&d_vox_perm_, sizeof(int2) * cap_vperm_));
         CK(cudaMalloc(&d_items_, sizeof(dev::Item) * cap_items_));
         CK(cudaMalloc(&d_stale_items_, sizeof(int) * cap_items_));
@@ -1366,8 +1366,8 @@ public:
             CK(cudaMalloc(&d_link_hist_, sizeof(int) * cap_bins_));
             CK(cudaMalloc(&d_link_base_, sizeof(int) * cap_bins_));
             if (!d_link_total_) {
-                CK(cudaMalloc(&d_link_total_, sizeof(int)));
-                CK(cudaMemsetAsync(d_link_total_, 0, sizeof(int), stream_));
+                CK(cudaMalloc(&d_link_total_, 2 * sizeof(int)));
+                CK(cudaMemsetAsync(d_link_total_, 0, 2 * sizeof(int), stream_));
             }
         }
         if (std::max<size_t>(1, links_total) > cap_perm_) {
@@ -1414,8 +1414,8 @@ public:
                 CK(cudaMalloc(&d_vox_hist_, sizeof(int) * cap_vbins_));
                 CK(cudaMalloc(&d_vox_base_, sizeof(int) * cap_vbins_));
                 if (!d_vox_total_) {
-                    CK(cudaMalloc(&d_vox_total_, sizeof(int)));
-                    CK(cudaMemsetAsync(d_vox_total_, 0, sizeof(int), stream_));
+                    CK(cudaMalloc(&d_vox_total_, 2 * sizeof(int)));
+                    CK(cudaMemsetAsync(d_vox_total_, 0, 2 * sizeof(int), stream_));
                 }
             }
             if (std::max<size_t>(1, vox_total) > cap_vperm_) {

@@ -434,6 +434,11 @@ __device__ __forceinline__ int bin_key(const Sim& S, int kind, int begin, int j)
     return kind == 0 ? LinkKey{S.lfl, begin}(j) : VoxelKey{S.vfl, begin}(j);
 }
 
+// Whether a launch takes the plain form for every element of a grouped list, total[1] of whose total[0]
+// elements are on it: an integer-pipe launch costs those block barriers and calls, 1.02-1.09 of the
+// plain kernels' time where nearly all are (this loop: 0.93-0.98), and saves the others about 0.4.
+__device__ __forceinline__ bool mostly_plain(const int* __restrict__ total) { return (long long)total[1] * 16 >= (long long)total[0] * 13; }
+
 // Takes an element that is ready for it off the plain form.
 __device__ __forceinline__ void leave_plain(const Sim& S, int kind, int at) {
     if (kind == 0) {
@@ -491,10 +496,15 @@ __global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, 
         const bool run = ctl[w.sim].status == 1;
         const Sim& S = sims[w.sim];
         const int n = w.end - w.begin;
-        const bool retry = kIntPipes && run && plain_retry(ctl[w.sim]);
+        const bool fresh = kIntPipes && run && ctl[w.sim].steps == 0;   // at rest, every element holds zeros
+        const bool retry = kIntPipes && run && !fresh && plain_retry(ctl[w.sim]);
         int cnt = 0;   // thread k < kOrderKeys: elements of key k
         for (int j0 = 0; j0 < n; j0 += blockDim.x) {
             const int j = j0 + threadIdx.x;
+            if (fresh && j < n) {
+                if (kind == 0) S.lfl[w.begin + j] |= LF_PLAIN;
+                else S.vfl[w.begin + j] |= VF_PLAIN;
+            }
             if (retry && j < n) leave_plain(S, kind, w.begin + j);
             const int kj = (run && j < n) ? bin_key(S, kind, w.begin, j) : -1;
 #pragma unroll
@@ -518,7 +528,7 @@ __global__ void __launch_bounds__(256) k_bin_hist(const Sim* __restrict__ sims, 
 __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const int* tickets, int n_links) {
     grid_wait();
     if (bins_settled(tickets, n_links)) return;
-    __shared__ int s_sum[1024];
+    __shared__ int s_sum[1024], s_plain;
     const BinList& L = blockIdx.x == 0 ? la : lb;   // one block per list
     const int* hist = L.hist;
     int* base = L.base;
@@ -533,15 +543,19 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const
         *k = r / win;
         return w * win + (r - *k * win);
     };
-    int sum = 0;
+    if (threadIdx.x == 0) s_plain = 0;
+    int sum = 0, plain = 0;
 #pragma unroll 8
     for (int e = e0; e < e1; e++) {
         int k;
         const int it = item_of(e, &k);
-        if (it < n_items) sum += hist[(size_t)it * kOrderKeys + k];
+        const int c = it < n_items ? hist[(size_t)it * kOrderKeys + k] : 0;
+        sum += c;
+        if (kIntPipes && k < kFormKeys) plain += c;
     }
     s_sum[threadIdx.x] = sum;
     __syncthreads();
+    if (plain) atomicAdd(&s_plain, plain);
     for (int off = 1; off < (int)blockDim.x; off <<= 1) {   // inclusive scan of the runs' sums
         const int v = (int)threadIdx.x >= off ? s_sum[threadIdx.x - off] : 0;
         __syncthreads();
@@ -558,7 +572,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(BinList la, BinList lb, const
             run += hist[(size_t)it * kOrderKeys + k];
         }
     }
-    if (threadIdx.x == blockDim.x - 1) *total = s_sum[blockDim.x - 1];
+    if (threadIdx.x == blockDim.x - 1) { total[0] = s_sum[blockDim.x - 1]; total[1] = s_plain; }
 }
 
 __global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sims, Ctl* ctl, BinList la, BinList lb, const int* tickets, int n_links) {
@@ -625,17 +639,12 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const Sim* __restrict__ sim
 constexpr int kLinkDefer = 48;          // a queue holds at most 31 + 16 links between rounds
 constexpr int kDeferPerWarp = 256;      // queues only with at least this many links per resident warp
 constexpr int kDeferRate = 256;         // queues while more than 1 link in kDeferRate changed mode
-// F: sums by DFMA (see Add in links_int.cuh); B: resident blocks an SM the registers are sized for.
-template <bool F, int B>
-__global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
-                                                                     const int* __restrict__ total, int cap, int n_slots, int* tickets,
-                                                                     int claim) {
-    grid_wait();
-    __shared__ int2 s_defer[GVX_STEP_BLOCK / 32][2][kLinkDefer];   // per warp: large-angle (0), small-angle (1)
-    const double one = F ? opaque_one() : 1.0;
-    // this step's queues of the kernels that follow, and the contact spill pool's records
-    if (blockIdx.x == 0 && threadIdx.x == 0) { tickets[1] = 0; tickets[2] = 0; tickets[3] = 0; tickets[4] = 0; }
-    const int n = min(*total, cap);
+
+// kInt: the integer-pipe form, with the plain one for the links that it leaves; else the plain form
+// alone.  F: sums by DFMA (see Add in links_int.cuh); B: resident blocks an SM the registers are sized for.
+template <bool kInt, bool F, int B>
+__device__ __forceinline__ void link_rounds(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm, int n, int n_slots, int* tickets,
+                                            int claim, double one, int2 (*s_defer)[2][kLinkDefer]) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     int2* q0 = s_defer[threadIdx.x >> 5][0];
@@ -668,7 +677,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
         }
         // the integer-pipe form is long straight-line code: a block's warps keep step through it
         // (here, and between its three parts below), so that one of them fetches it for all
-        if (kIntPipes ? !__syncthreads_or(src != 2) : src == 2) break;
+        if (kInt ? !__syncthreads_or(src != 2) : src == 2) break;
         int2 e = make_int2(-1, -1);
         if (src == 2) {
         } else if (src < 0) {
@@ -689,18 +698,18 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
         LinkOrient o;
         IntPipes<F> ip(one);
         bool plain = false;      // this link takes the plain form (and is not deferred)
-        if (kIntPipes) {
+        if (kInt) {
             if (act) {
                 const Sim& S = sims[e.x];
                 const uint8_t fl = S.lfl[e.y];
                 act = !(fl & LF_GONE) && !((S.flags & SF_FIXEDMAT) && fixed_link(S, e.y));
-                plain = (fl & LF_PLAIN) || ctl[e.x].steps == 0;   // at rest before step 0, every link holds zeros
+                plain = fl & LF_PLAIN;
             }
             const bool both = __ballot_sync(0xffffffffu, act && !plain) != 0;
             if (act) {
                 const Sim& S = sims[e.x];
                 const uint8_t fl = S.lfl[e.y];
-                if (plain && both && (fl & LF_PLAIN)) plain = !link_ready(S, e.y, fl);
+                if (plain && both) plain = !link_ready(S, e.y, fl);
                 if (!plain) {
                     link_orient_int(ip, S, e.y, fl, &o);
                     plain = !ip.ok();
@@ -726,7 +735,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
             }
             act = act && !defer;
         }
-        if (kIntPipes) {
+        if (kInt) {
             bool div = false;
             LinkPose p;
             __syncthreads();
@@ -740,11 +749,29 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
         } else if (act) {
             Ctl& c = ctl[e.x];
             bool div = false;
+            const uint8_t form = kIntPipes ? sims[e.x].lfl[e.y] & LF_PLAIN : 0;   // stays what it was
             link_finish(sims[e.x], e.y, c.dt, o, &div);
+            if (form) sims[e.x].lfl[e.y] |= form;
             if (div) c.diverged = 1;
         }
     }
     if (lane == 0 && switched) atomicAdd(&tickets[5], switched);
+}
+
+template <bool F, int B>
+__global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
+                                                                     const int* __restrict__ total, int cap, int n_slots, int* tickets,
+                                                                     int claim) {
+    grid_wait();
+    __shared__ int2 s_defer[GVX_STEP_BLOCK / 32][2][kLinkDefer];   // per warp: large-angle (0), small-angle (1)
+    const double one = F ? opaque_one() : 1.0;
+    // this step's queues of the kernels that follow, and the contact spill pool's records
+    if (blockIdx.x == 0 && threadIdx.x == 0) { tickets[1] = 0; tickets[2] = 0; tickets[3] = 0; tickets[4] = 0; }
+    const int n = min(*total, cap);
+    if (kIntPipes && !mostly_plain(total))
+        link_rounds<true, F, B>(sims, ctl, perm, n, n_slots, tickets, claim, one, s_defer);
+    else
+        link_rounds<false, F, B>(sims, ctl, perm, n, n_slots, tickets, claim, one, s_defer);
 }
 
 // Overlap test and repelling force for one voxel pair (CVX_Collision::updateContactForce,
@@ -1692,6 +1719,62 @@ __device__ __noinline__ void sim_control(const Sim& S, Ctl& c, bool div, double 
     if (stop) c.status = 2;
 }
 
+// kInt and F as in link_rounds.
+template <bool kInt, bool F>
+__device__ __forceinline__ void voxel_rounds(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm, int n, int n_slots, int* tickets,
+                                             int claim, double one) {
+    const int lane = threadIdx.x & 31;
+    int k = 0, k1 = 0;           // the claimed chunk: next round's first voxel, its end
+    bool more = true;            // chunks may remain
+    for (;;) {
+        if (k >= k1 && more) {
+            int chunk = 0;
+            if (lane == 0) chunk = atomicAdd(&tickets[2], 1);
+            chunk = __shfl_sync(0xffffffffu, chunk, 0);
+            k = chunk * claim;
+            k1 = min(n, k + claim);
+            if (k >= n) more = false;
+        }
+        // a block's warps keep step through the integer-pipe form (see k_links)
+        if (kInt ? !__syncthreads_or(k < k1) : k >= k1) break;
+        int2 e = make_int2(-1, -1);
+        if (k + lane < k1) e = __ldg(perm + k + lane);
+        k += 32;
+        // e.x >= n_slots: none, or never (the grouping lists running slots)
+        bool act = (unsigned)e.x < (unsigned)n_slots;
+        if (act) {
+            const Ctl& c = ctl[e.x];
+            act = c.status == 1 && !c.diverged && c.dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv;
+        }
+        uint32_t fl = 0;
+        bool plain = false;
+        if (kInt) {
+            if (act) {
+                fl = sims[e.x].vfl[e.y];
+                plain = (fl & VF_PLAIN) || always_plain(sims[e.x].flags, fl);
+            }
+            const bool both = __ballot_sync(0xffffffffu, act && !plain) != 0;
+            if (plain && both && !always_plain(sims[e.x].flags, fl)) plain = !voxel_ready(sims[e.x], e.y, fl);
+        }
+        if (act) {
+            const Ctl& c = ctl[e.x];
+            const float dt = c.dt;
+            const Sim& S = sims[e.x];
+            StepTimes st;
+            st.t_now = c.t; st.t_next = c.t + dt; st.t_cycles = c.t_cycles; st.angle = c.recent_angle;
+            st.closeness = c.closeness; st.close_pairs = c.num_close_pairs; st.hits = c.hit_count;
+            int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
+            int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
+            if (kInt) {
+                if (!plain) plain = !voxel_update_int<F>(S, e.y, fl, dt, st, S.flags, one, hnext, moved);
+                if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
+            } else {
+                voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, moved);
+            }
+        }
+    }
+}
+
 template <bool F>
 __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxels(const Sim* __restrict__ sims, Ctl* ctl, const int2* __restrict__ perm,
                                                                        const int* __restrict__ total, int cap, int n_slots, int* tickets,
@@ -1708,56 +1791,10 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, GVX_VOXELS_MIN_BLOCKS) k_voxel
         tickets[7] = 0;            // this step's watch-list passes are done: k_sim_end lists the next
     }
     const int n = min(*total, cap);
-    const int lane = threadIdx.x & 31;
-    int k = 0, k1 = 0;           // the claimed chunk: next round's first voxel, its end
-    bool more = true;            // chunks may remain
-    for (;;) {
-        if (k >= k1 && more) {
-            int chunk = 0;
-            if (lane == 0) chunk = atomicAdd(&tickets[2], 1);
-            chunk = __shfl_sync(0xffffffffu, chunk, 0);
-            k = chunk * claim;
-            k1 = min(n, k + claim);
-            if (k >= n) more = false;
-        }
-        // a block's warps keep step through the integer-pipe form (see k_links)
-        if (kIntPipes ? !__syncthreads_or(k < k1) : k >= k1) break;
-        int2 e = make_int2(-1, -1);
-        if (k + lane < k1) e = __ldg(perm + k + lane);
-        k += 32;
-        // e.x >= n_slots: none, or never (the grouping lists running slots)
-        bool act = (unsigned)e.x < (unsigned)n_slots;
-        if (act) {
-            const Ctl& c = ctl[e.x];
-            act = c.status == 1 && !c.diverged && c.dt != 0.0f && (unsigned)e.y < (unsigned)sims[e.x].nv;
-        }
-        uint32_t fl = 0;
-        bool plain = false;
-        if (kIntPipes) {
-            if (act) {
-                fl = sims[e.x].vfl[e.y];
-                plain = (fl & VF_PLAIN) || always_plain(sims[e.x].flags, fl) || ctl[e.x].steps == 0;
-            }
-            const bool both = __ballot_sync(0xffffffffu, act && !plain) != 0;
-            if (plain && both && (fl & VF_PLAIN) && !always_plain(sims[e.x].flags, fl)) plain = !voxel_ready(sims[e.x], e.y, fl);
-        }
-        if (act) {
-            const Ctl& c = ctl[e.x];
-            const float dt = c.dt;
-            const Sim& S = sims[e.x];
-            StepTimes st;
-            st.t_now = c.t; st.t_next = c.t + dt; st.t_cycles = c.t_cycles; st.angle = c.recent_angle;
-            st.closeness = c.closeness; st.close_pairs = c.num_close_pairs; st.hits = c.hit_count;
-            int* hnext = (S.flags & SF_COLLIDE) ? S.hash_head + (size_t)(c.hash_parity ^ 1) * S.hash_size : nullptr;
-            int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
-            if (kIntPipes) {
-                if (!plain) plain = !voxel_update_int<F>(S, e.y, fl, dt, st, S.flags, one, hnext, moved);
-                if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
-            } else {
-                voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, moved);
-            }
-        }
-    }
+    if (kIntPipes && !mostly_plain(total))
+        voxel_rounds<true, F>(sims, ctl, perm, n, n_slots, tickets, claim, one);
+    else
+        voxel_rounds<false, F>(sims, ctl, perm, n, n_slots, tickets, claim, one);
 }
 
 // The end of a step for each simulation of the batch, one block each: on cycle steps the
