@@ -283,7 +283,7 @@ public:
     dev::Sim* d_sims_ = nullptr;
     dev::Ctl* d_ctl_ = nullptr;
     std::vector<SimRec*> slot_owner_;
-    // queue tickets of the step kernels (0 links, 1 contacts, 2 voxels, 3 signals) and the
+    // queue tickets of the step kernels (0 links, 2 voxels, 3 signals; 1 is not used) and the
     // contact spill pool's record count of the step
     static constexpr int kTickets = 8, kSpillTicket = 4;
     int* d_tickets_ = nullptr;

@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(GVX_STEP_BLOCK, B) k_links(const Sim* __restri
     __shared__ int2 s_defer[GVX_STEP_BLOCK / 32][2][kLinkDefer];   // per warp: large-angle (0), small-angle (1)
     const double one = F ? opaque_one() : 1.0;
     // this step's queues of the kernels that follow, and the contact spill pool's records
-    if (blockIdx.x == 0 && threadIdx.x == 0) { tickets[1] = 0; tickets[2] = 0; tickets[3] = 0; tickets[4] = 0; }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { tickets[2] = 0; tickets[3] = 0; tickets[4] = 0; }
     const int n = min(*total, cap);
     if (kIntPipes && !mostly_plain(total))
         link_rounds<true, F, B>(sims, ctl, perm, n, n_slots, tickets, claim, one, s_defer);
