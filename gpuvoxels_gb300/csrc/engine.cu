@@ -320,7 +320,7 @@ public:
     static constexpr int kRegroupSmall = 64, kYoungSteps = 16;
     int young_left_ = 0;   // steps until no simulation of the running batch is in its first kYoungSteps
     void set_young(int64_t youngest) { young_left_ = (int)std::max<int64_t>(0, kYoungSteps - youngest); }
-    size_t batch_links_ = 0, batch_voxels_ = 0;
+    size_t batch_links_ = 0, batch_voxels_ = 0, batch_surface_ = 0;   // batch_surface_: surface voxels of the contact items
     int sm_count_ = 152;
     int profiling_ = 0;
     KernelSet ks_ = kernelset_exact();
@@ -1376,6 +1376,7 @@ public:
             cap_perm_ = std::max(std::max<size_t>(1, links_total), 2 * cap_perm_);
             CK(cudaMalloc(&d_link_perm_, sizeof(int2) * cap_perm_));
         }
+        batch_surface_ = 0;
         std::vector<std::pair<int, int>> contact_items(slots.size(), std::make_pair(0, 0));   // per batch entry: first, count
         for (size_t k = 0; k < slots.size(); k++) {
             const int s = slots[k];
@@ -1385,6 +1386,7 @@ public:
             const int ns = contact_list_size(r->w);
             if (!r->w.desc.collisions || ns == 0) continue;
             any_collide_ = true;
+            batch_surface_ += (size_t)ns;
             if (watches(r->w.desc)) any_watch_ = true;
             const int chunk = 128;   // at most 128 surface voxels an item (the watch passes' work units rely on it)
             const int first = (int)items.size() - n_link_items_;
@@ -1536,7 +1538,7 @@ public:
         // the watch-list passes: a persistent grid of 256-thread blocks over the listed items' work units
         if (any_watch_) ks_.watch(4 * sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_, d_stale_items_, d_tickets_, d_batch_slots_,
                                   n_batch_);
-        if (any_collide_) ks_.contacts(sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_);
+        if (any_collide_) ks_.contacts(sm_count_, st, d_sims_, d_ctl_, ci, n_contact_items_, batch_surface_);
         if (n_attach_) ks_.attach(st, d_sims_, d_ctl_, d_attach_slots_, n_attach_);
         if (prof) cudaEventRecord(evk_[2], st);
         if (prof) cudaEventRecord(evk_[3], st);

@@ -1245,12 +1245,15 @@ __device__ void voxel_contacts_watch(const Sim& S, int v, int si, Ctl& c, int g,
 //
 // Bound: latency.  Every partner is two dependent reads (list, position) and for the few that touch the
 // state of both, after five reads a voxel; a lane that walks its list alone takes as long as the longest
-// list.  Eight lanes a voxel where the warps are few: 37 -> 16 us for a settled 12^3 creature, 55 -> 20
-// for a 24^3 one, 57 -> 33 for a 40^3 one (31,000 surface voxels).  In a large batch they repeat the
-// reads a voxel for four voxels instead of 32 (249,000 surface voxels: 219 us against 117 settled), so
-// kContactWide surface voxels and fewer take them.  Seven blocks an SM: the integer-pipe pair test
-// at 96 registers and five blocks took 135 us there, at 64 and eight 119; the FP64 test 141.
-constexpr int kContactWide = 32768;
+// list.  Eight lanes a voxel where the warps are few; in a large batch they repeat the reads a voxel for four
+// voxels instead of 32.  Contact and watch passes of settled bodies with eight lanes and one, us: 12^3 (800
+// surface voxels) 18 and 35, 300 of 4^3 (8,000) 20 and 27, 40^3 (30,500) 27 and 42, two of 36^3 (44,500) 33 and
+// 45, two of 40^3 (61,000) 41 and 43 (fresh 31 and 29), four (122,500) 70 and 59, eight (245,000) 127 and 96.
+// So kContactWide surface voxels and fewer take eight, in kContactWideItems items at most: of the
+// units of more items than that most are empty (1,200 of 4^3, 31,500 surface voxels: 43 and 39).
+// Seven blocks an SM: with one lane the integer-pipe pair test at 96 registers and five blocks took 135 us
+// over 249,000 surface voxels, at 64 and eight 119, the FP64 test 141, this 117.
+constexpr int kContactWide = 49152, kContactWideItems = 1024;
 template <int G>
 __global__ void __launch_bounds__(128, 7) k_contacts(const Sim* __restrict__ sims, Ctl* ctl, const Item* __restrict__ items, int n_items) {
     grid_wait();
@@ -2143,9 +2146,10 @@ inline void l_links(int g, int b, cudaStream_t s, const Sim* sims, Ctl* ctl, con
     if (kIntPipes && depth == 2) k = k_links<kIntPipes, kIntPipes ? 3 : GVX_LINKS_MIN_BLOCKS>;
     step_launch(k, g, b, s, sims, ctl, perm, total, cap, n_slots, tk, claim);
 }
-inline void l_contacts(int sms, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n) {
-    // n items of at most 128 surface voxels; four warps a block
-    if (n <= kContactWide / 128) step_launch(k_contacts<8>, std::max(1, std::min(8 * n, 8 * sms)), 128, s, sims, ctl, it, n);
+inline void l_contacts(int sms, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n, size_t surface) {
+    // n items of at most 128 surface voxels, `surface` in all; four warps a block
+    if (surface <= (size_t)kContactWide && n <= kContactWideItems)
+        step_launch(k_contacts<8>, std::max(1, std::min(8 * n, 8 * sms)), 128, s, sims, ctl, it, n);
     else step_launch(k_contacts<1>, std::max(1, std::min(n, 16 * sms)), 128, s, sims, ctl, it, n);
 }
 inline void l_watch(int g, cudaStream_t s, const Sim* sims, Ctl* ctl, const Item* it, int n_items, const int* stale, const int* tk,

@@ -19,7 +19,8 @@ struct KernelSet {
     // depth: 0 not every resident warp has a chunk, 1 every one has, 2 (links) every one has many
     void (*links)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
                   int n_slots, int* tickets, int claim, int depth);
-    void (*contacts)(int sm_count, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n_items);
+    // the contact pass over n items that hold `surface` surface voxels
+    void (*contacts)(int sm_count, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const dev::Item* items, int n_items, size_t surface);
     void (*voxels)(int grid, int block, cudaStream_t s, const dev::Sim* sims, dev::Ctl* ctl, const int2* perm, const int* total, int cap,
                    int n_slots, int* tickets, int claim, int depth);
     // the end of the step for n simulations (slot list): centre-of-mass sample, time, stop;
