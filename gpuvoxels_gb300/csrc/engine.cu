@@ -1494,9 +1494,10 @@ public:
         const size_t per_sm = (size_t)ks_.resident_blocks(which, block), most = (size_t)block / 32;   // blocks an SM, warps a block
         const size_t want = (chunks + sms - 1) / sms;                                                // warps an SM
         // From kDeepRounds chunks a resident warp on, k_links takes its build for three blocks an SM (80
-        // registers): 512 creatures (19 chunks a warp) 24.4 -> 23.3 ms a pass, a slab (33) 18.1 -> 17.7;
-        // with five chunks a warp the longer tail costs more than it gives (128 creatures 7.29 -> 7.36 ms,
-        // eight colliding ones 8.25 -> 8.41).
+        // registers).  Time a step with three blocks over that with two, settled, by chunks a warp of two blocks:
+        // creatures 2.3: 1.03, 3.2: 1.02, 5.3: 0.985, 7.6: 0.98, 10.6: 0.98, 19.7: 0.985; eight self-colliding ones
+        // 4.8: 1.02; solid bodies 1.7: 1.05, 4.2: 0.93, 9.9 and more: 0.97.  Below 10 it is either side of 1.
+        // (With 1.3 and 1.5 chunks, which three blocks hold in one round, it is 0.91; the rule leaves that out.)
         constexpr size_t kDeepRounds = 10;
         if (which == 0 && want >= kDeepRounds * most * per_sm) return {(int)(sms * ks_.resident_blocks(2, block)), block, 2};
         if (want >= most * per_sm) return {(int)(sms * per_sm), block, 1};
