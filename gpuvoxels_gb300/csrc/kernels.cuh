@@ -1595,10 +1595,11 @@ __device__ __forceinline__ void voxel_update(const Sim& S, int v, float dt, cons
 namespace gvx {
 namespace GVX_KNS {
 
-// The plain form of a voxel's step (see link_plain).
+// The plain form of a voxel's step, out of line (see link_plain): one copy of it a kernel, which with its
+// formulas' stacks takes 700 bytes of local memory a thread.  (Inlined into the loop of the plain form as
+// well it was 1,200, above the context's stack limit: raising that took 9 ms of a process's first step.)
 __device__ __noinline__ void voxel_plain(const Sim& S, int v, float dt, const StepTimes& st, int* hash_next_table, int* watch_moved) {
     voxel_update(S, v, dt, st, S.flags, nullptr, hash_next_table, watch_moved);
-    S.vfl[v] |= VF_PLAIN;
 }
 
 __device__ __forceinline__ double block_sum(double x, double* red) {
@@ -1770,7 +1771,12 @@ __device__ __forceinline__ void voxel_rounds(const Sim* __restrict__ sims, Ctl* 
             int* moved = (S.flags & SF_WATCH) ? &ctl[e.x].col_moved : nullptr;
             if (kInt) {
                 if (!plain) plain = !voxel_update_int<F>(S, e.y, fl, dt, st, S.flags, one, hnext, moved);
-                if (plain) voxel_plain(S, e.y, dt, st, hnext, moved);
+                if (plain) {
+                    voxel_plain(S, e.y, dt, st, hnext, moved);
+                    S.vfl[e.y] |= VF_PLAIN;
+                }
+            } else if (kIntPipes) {
+                voxel_plain(S, e.y, dt, st, hnext, moved);   // VF_PLAIN stays what it was
             } else {
                 voxel_update(S, e.y, dt, st, S.flags, nullptr, hnext, moved);
             }
