@@ -1810,7 +1810,12 @@ public:
         tc.mark("step: drive");
         exact_steps_ = -1;
         if (int e2 = end_fixed_steps(slots, err)) return e2;
-        if (e) return e;
+        if (e) {   // drive has not read how far the simulations came
+            std::string e3;
+            if (read_ctls(lo, hi, &cs, &e3) == 0)
+                for (auto* r : act) r->status = cs[(size_t)(r->slot - lo)].status;
+            return e;
+        }
         for (auto* r : act) {   // what end_fixed_steps leaves on the device
             const int st = cs[(size_t)(r->slot - lo)].status;
             r->status = st == SIM_DONE ? SIM_IDLE : st;
