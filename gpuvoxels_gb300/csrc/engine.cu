@@ -2042,9 +2042,23 @@ public:
             queue_.push_front(big);
             lane_first = true;
         }
+        // a simulation that is running already (its id submitted again) waits in the queue until it is done:
+        // listed twice its voxels would be updated by two threads of a step, and finished after its release
+        std::unordered_set<int64_t> running(active_.begin(), active_.end());
+        std::vector<int64_t> waiting;
+        struct Requeue {   // puts them back in their order on every way out
+            std::deque<int64_t>& q; std::vector<int64_t>& w;
+            ~Requeue() { q.insert(q.begin(), w.begin(), w.end()); }
+        } requeue{queue_, waiting};
         while (!queue_.empty()) {
             SimRec* r = find(queue_.front());
             if (!r) { queue_.pop_front(); lane_first = false; continue; }
+            if (!running.insert(r->id).second) {
+                waiting.push_back(r->id);
+                queue_.pop_front();
+                lane_first = false;
+                continue;
+            }
             const bool in_lane = lane_first && admitted.empty();
             if (!in_lane && serve_max_voxels_ > 0 && !(active_.empty() && admitted.empty()) &&
                 active_voxels + r->w.nv > serve_max_voxels_)
