@@ -315,8 +315,11 @@ public:
     // their links and voxels are regrouped only when the batch changes and at the start of
     // every graph replay, or after as many steps, and before steps 4, 8 and 16 of the youngest simulation
     // (elements leave the plain form when they are grouped).  The steps before the 16th are launched
-    // one by one: a graph of theirs would be replayed for later ones.
-    static constexpr size_t kRegroupEveryStepLinks = 200000;
+    // one by one: a graph of theirs would be replayed for later ones.  A batch with less than a warp of links for
+    // each quarter of the SMs leaves out step 8 (a grouping takes it 21 us): steps 4 to 15 of a 10^3 body of equal
+    // phases take 48 us each without it and 64 with it, of a 10^3 creature 58 and 59; with more links, 64
+    // equal-phase cantilevers' take 7 % longer without it, other bodies' 2 % less to 2 % more.
+    static constexpr size_t kRegroupEveryStepLinks = 200000, kRegroupTwiceLinks = 32 * 4 * 152;
     static constexpr int kRegroupSmall = 64, kYoungSteps = 16;
     int young_left_ = 0;   // steps until no simulation of the running batch is in its first kYoungSteps
     void set_young(int64_t youngest) { young_left_ = (int)std::max<int64_t>(0, kYoungSteps - youngest); }
@@ -1513,7 +1516,7 @@ public:
         const dev::Item* vi = d_items_ + n_link_items_ + n_contact_items_;
         const bool large = batch_links_ >= kRegroupEveryStepLinks;
         const int age = kYoungSteps - young_left_;   // of the youngest simulation
-        const bool regroup = bins_dirty_ || bin_phase_ % (large ? bin_every_ : kRegroupSmall) == 0 || (!large && (age == 4 || age == 8));
+        const bool regroup = bins_dirty_ || bin_phase_ % (large ? bin_every_ : kRegroupSmall) == 0 || (!large && (age == 4 || (age == 8 && batch_links_ >= kRegroupTwiceLinks)));
         const bool maybe = !regroup && large && bin_adapts_ && bin_phase_ % 2 == 0;   // decided on the device
         if (regroup || maybe) {
             // links and voxels grouped together (the voxel keys come from the last voxel
