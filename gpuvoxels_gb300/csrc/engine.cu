@@ -1510,7 +1510,7 @@ public:
 
     // One step of the batch; returns the number of kernels it launched.
     int launch_step(cudaStream_t st, bool prof) {
-        int launched = 3 + (any_collide_ ? 1 : 0) + (any_watch_ ? 3 : 0) + (any_signals_ ? 1 : 0) + (n_attach_ ? 1 : 0);
+        int launched = 3 + (any_collide_ ? 1 : 0) + (any_watch_ ? 1 : 0) + (any_signals_ ? 1 : 0) + (n_attach_ ? 1 : 0);
         const dev::Item* li = d_items_;
         const dev::Item* ci = d_items_ + n_link_items_;
         const dev::Item* vi = d_items_ + n_link_items_ + n_contact_items_;

@@ -20,3 +20,16 @@ def test_regrouping_period(monkeypatch, every, groupings):
         assert ctx.info(sim).num_link >= 200000
         ctx.step(sim, 16)
         assert ctx.timing()["launches"] == 3 * 16 + 3 * groupings
+
+
+def test_launch_count_with_contacts():
+    """A self-colliding body's step is five kernels (links, watch lists, contacts, voxels, control), and the
+    grouping three more: the count a call reports is that of the kernels it launched."""
+    import gpuvoxels_gb300 as g
+    from gpuvoxels_gb300 import synth
+    mats = [dict(E=1e5, rho=1000.0, nu=0.35, cte=0.01, mus=1.0, muk=0.5)]
+    with g.Context(0, 256 << 20) as ctx:
+        sim = ctx.load_vxa(synth.random_creature(2, (6, 6, 6), 0.6, mats, collision=True, expansion=False).vxa)
+        ctx.step(sim, 40)
+        ctx.step(sim, 10)
+        assert ctx.timing()["launches"] == 5 * 10 + 3
