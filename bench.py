@@ -73,22 +73,22 @@ def measured_peaks():
 # dram__bytes_write.sum / links).  profiles/fp64_counts_by_workload.md has the captures.
 FP64_COUNTS = {
     # batch of 512 creatures, step 288 (the settled window the line's value is timed over)
-    "batch": dict(per_link=308699104 / 1627115, per_voxel=86921632 / 844972,
-                  lanes_link=308699104 / 10684910, lanes_voxel=86921632 / 3139438,
-                  traffic_per_link=(431895040 + 671297024) / 1627115, source="ncu, 512-creature batch, step 288"),
+    "batch": dict(per_link=308667296 / 1627115, per_voxel=86921312 / 844972,
+                  lanes_link=308667296 / 10621610, lanes_voxel=86921312 / 3138264,
+                  traffic_per_link=(417531904 + 627112448) / 1627115, source="ncu, 512-creature batch, step 288"),
     # 8 of the 64 collision creatures, mean of steps 201, 1001 and 1901 (the 2,000 timed steps)
-    "collide": dict(per_link=(70586144 + 64533024 + 63018592) / 3 / 373621,
-                    per_voxel=(30746112 + 27282656 + 26794624) / 3 / 249183,
-                    lanes_link=(70586144 + 64533024 + 63018592) / (2406790 + 2158689 + 2120036),
-                    lanes_voxel=(30746112 + 27282656 + 26794624) / (1132672 + 1044085 + 1047985),
-                    traffic_per_link=(191341312 + 188014560 + 188793472) / 3 / 373621,
+    "collide": dict(per_link=(70580288 + 64528608 + 63009312) / 3 / 373621,
+                    per_voxel=(30745536 + 27284064 + 26794816) / 3 / 249183,
+                    lanes_link=(70580288 + 64528608 + 63009312) / (2395196 + 2150612 + 2102133),
+                    lanes_voxel=(30745536 + 27284064 + 26794816) / (1132672 + 1044085 + 1047985),
+                    traffic_per_link=(190146560 + 188150016 + 187610880) / 3 / 373621,
                     source="ncu, 8 collision creatures 40^3, mean of steps 201, 1001, 1901"),
     # a 100x100x50 slab, mean of steps 201, 1001 and 1901
-    "slab": dict(per_link=(340309184 + 339917792 + 339795712) / 3 / 1480000,
-                 per_voxel=(54041344 + 53835072 + 53802912) / 3 / 500000,
-                 lanes_link=(340309184 + 339917792 + 339795712) / (11182512 + 11179330 + 11174281),
-                 lanes_voxel=(54041344 + 53835072 + 53802912) / (1713486 + 1701517 + 1700288),
-                 traffic_per_link=(663611392 + 667149568 + 668494080) / 3 / 1480000,
+    "slab": dict(per_link=(340301696 + 339903488 + 339778464) / 3 / 1480000,
+                 per_voxel=(54041632 + 53835136 + 53802816) / 3 / 500000,
+                 lanes_link=(340301696 + 339903488 + 339778464) / (11169821 + 11154305 + 11143115),
+                 lanes_voxel=(54041632 + 53835136 + 53802816) / (1713486 + 1701517 + 1700288),
+                 traffic_per_link=(631078656 + 631851840 + 630645504) / 3 / 1480000,
                  source="ncu, 100x100x50 slab, mean of steps 201, 1001, 1901"),
 }
 # steps a whole run of each workload takes (the batch: 0.5 s simulated at its creatures' time steps)
