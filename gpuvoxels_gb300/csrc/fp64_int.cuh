@@ -185,8 +185,8 @@ GVX_FP64I double times_zero(double k, double z) {   // k * z
 // no lane active as with 32.)
 //
 // Why: measured on GB300 (2 blocks of 256 threads an SM, four independent chains a thread), a
-// warp's DADD or DMUL takes 77 cycles of its quarter of the SM, a division 548, a square root
-// 572, and the integer pipes run beside it: a product formed here takes 42-50 cycles of issue,
+// warp's DADD or DMUL takes about 80 cycles of its quarter of the SM (77 in this probe, 80 in the one of
+// Add in links_int.cuh), a division 548, a square root 572, and the integer pipes run beside it: a product formed here takes 42-50 cycles of issue,
 // and product-and-add pairs (product here, sum on the FP64 pipe) 82 cycles a pair against 154,
 // two products and an add 97 against 231.
 constexpr uint32_t kOutOfBand = 0xC0000000u;

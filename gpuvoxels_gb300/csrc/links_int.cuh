@@ -1,17 +1,18 @@
 // The link update with its products, quotients and square roots on the integer pipes.
 //
-// Bound: GB300's FP64 pipe.  A warp's FP64 instruction occupies it for 77 cycles of an SM
-// quarter whatever its active lanes, and a link took about 400 of them while the integer pipes
+// Bound: GB300's FP64 pipe.  A warp's FP64 addition occupies it for about 80 cycles of an SM
+// quarter (see Add) whatever its active lanes, and a link took about 400 of them while the integer pipes
 // issued in one cycle of ten.  Here the FP64 pipe keeps the additions (and the libm calls);
 // multiplications, divisions, roots and conversions are the exact integer forms of
 // fp64_int.cuh, so every stored value has the bits of the plain form (link_orient and
 // link_finish in kernels.cuh).  Those forms hold for operands in their exponent band; a link
 // with any other operand (zeros in a body's first steps, exact symmetries, overflow) is found
-// by the `rare` word at the end and taken again by the plain form.  In-place state is therefore
+// by the `rare` word at the end and taken again by the plain form, on which it then stays (LF_PLAIN).  In-place state is therefore
 // written only after that check; the direction slots, which are outputs alone, before it.
 //
 // k_links on 128 settled creatures (371 k links): 329 -> 218 us, 4.98 -> 2.35 M FP64 warp
-// instructions beside 64 M integer ones (issue slots 11 -> 31 % used).  Leaving any group of the
+// instructions beside 64 M integer ones (issue slots 11 -> 31 % used); with elements grouped by form, 337 -> 208
+// us over another 128 (375 k links).  Leaving any group of the
 // products (orientation, damping, a rotation) on the FP64 pipe measured 1.5-6 % slower passes.
 //
 // The terms that the two angle modes make exactly zero (see beam_forces) are left out: their
@@ -25,7 +26,7 @@ namespace GVX_KNS {
 // A double whose sums and differences, with F set, are formed as x * 1 + y by DFMA, with the 1 in a
 // register that the compiler cannot see through.  Exactly x + y, and faster where the whole chip is
 // busy: with all four quarters of an SM at it a DFMA of three registers takes 17.0 cycles of the SM, a
-// DADD or DMUL (or a DFMA with a constant or uniform operand) 20.1.  A quarter alone takes 69 for either,
+// DADD or DMUL (or a DFMA with a constant or uniform operand) 20.1, 80 of a quarter's.  A quarter alone takes 69 for either,
 // and the register and the negations cost small batches 1-2 %, so those take F clear.
 template <bool F>
 struct Add {

@@ -101,7 +101,8 @@ int vx3_set_external(vx3_ctx* ctx, vx3_sim_id id, int voxel, int dof_fixed, cons
                      const double translate[3], const double rotate[3]);
 
 /* Replaces VX3_SimulationManager::start() for a batch (VX3_SimulationManager.cu:138-155):
- * runs every listed simulation until its StopConditionFormula holds (or max_steps, 0 = 1e6). */
+ * runs every listed simulation until its StopConditionFormula holds (or max_steps, 0 = 1e6).  An id
+ * listed more than once, here and in vx3_step, is one simulation. */
 int vx3_run(vx3_ctx* ctx, const vx3_sim_id* ids, int n, int mode, int64_t max_steps);
 /* Replaces n calls of VX3_VoxelyzeKernel::doTimeStep() (VX3_VoxelyzeKernel.cu:237-359). */
 int vx3_step(vx3_ctx* ctx, const vx3_sim_id* ids, int n, int mode, int64_t steps);
@@ -109,7 +110,8 @@ int vx3_step(vx3_ctx* ctx, const vx3_sim_id* ids, int n, int mode, int64_t steps
 /* Serving pair (no reference counterpart beyond the dir-watch daemon, Executables/vx3_node_daemon.cu:16-66):
  * submit queues a loaded simulation with a horizon in steps; poll admits queued simulations as
  * the HBM budget allows, advances all admitted ones by `chunk_steps`, retires finished ones and
- * returns up to `max` results (the count, or a negative status). */
+ * returns up to `max` results (the count, or a negative status).  A simulation submitted again while it
+ * runs is admitted when it is done, and runs afresh. */
 int vx3_submit(vx3_ctx* ctx, vx3_sim_id id, int64_t horizon_steps);
 int vx3_poll(vx3_ctx* ctx, vx3_result* out, int max, int chunk_steps);
 int vx3_pending(vx3_ctx* ctx);
