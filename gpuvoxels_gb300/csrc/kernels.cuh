@@ -308,12 +308,14 @@ __device__ __noinline__ bool link_plain(const Sim& S, int l, float dt, bool* swi
 // zeros sent them there are well inside the band (the products of two such are in band too).  A warp with
 // lanes on either form runs both.  So that is looked at when elements are grouped, where those that
 // change forms change warps as well, and between groupings in warps that run both forms anyway.  Groupings
-// look at a simulation's elements up to its 16th step and then in one of 16 steps at most: an element
-// that fails for a reason which the look does not see pays for both forms no oftener.
+// look at a simulation's elements before steps 4 to 16 and then in one of 16 steps at most: an element
+// that fails for a reason which the look does not see pays for both forms no oftener.  (Of a random
+// creature's links 45-63 % hold an exact zero before step 1, 0.01-1 % before step 4; taken off step by
+// step before that, they cost a small creature's steps 2 and 3, called singly, 68 and 71 us, not 60 and 62.)
 // Against the plain kernels alone, steps 4 to 15 of a body whose zeros last or recede slowly (equal
 // phases, 110,592 voxels) went from 1.33 of their time, with a trial every step, to 1.07 (the rest: barriers
 // and calls around the plain form), 64 cantilevers' steps from 1.04-1.07 to 0.72.
-__device__ __forceinline__ bool plain_retry(const Ctl& c) { return c.steps <= 16 || c.steps - c.plain_at >= 16; }
+__device__ __forceinline__ bool plain_retry(const Ctl& c) { return c.steps >= 4 && (c.steps <= 16 || c.steps - c.plain_at >= 16); }
 __device__ __forceinline__ bool sizable(double x) { return (fp64i::hi32(x) & 0x7FF00000u) - ((1023u - 110u) << 20) < (220u << 20); }   // 2^-110..2^110
 
 // The rotations of both voxels, and of the link's last pose what its mode does not make zero.
